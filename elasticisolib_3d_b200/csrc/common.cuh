@@ -50,6 +50,7 @@ struct GridConst {
   // y-slab of a decomposed grid: local plane y is global plane y + yOff of a grid of nyTaper
   // planes, whose y faces carry the sponge (a whole grid: yOff = 0, nyTaper = ny)
   int yOff, nyTaper;
+  int pz;  // row pitch of the fields in floats: nz, or nz rounded up (the paired stepper's padded rows)
 };
 
 #ifdef __CUDACC__

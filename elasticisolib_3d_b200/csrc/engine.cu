@@ -56,6 +56,16 @@ struct Fields9 {
   float* p[NCOMP] = {};
 };
 
+// Injected points binned by the paired stepper's CTAs (kAcqCount/Scan/Fill), kept between calls for
+// their memory only: every call bins its own positions.
+struct AcqTable {
+  int* row = nullptr;     // owners + 1
+  int* cursor = nullptr;
+  AcqEntry* entries = nullptr;
+  size_t rowCap = 0, entryCap = 0;
+  int n = 0;              // points of the current call (0: none)
+};
+
 struct Context {
   ContextDesc d;
   cudaStream_t st = nullptr;     // stream all work is queued on
@@ -82,6 +92,19 @@ struct Context {
   unsigned* posFlag = nullptr;  // device word of the position-table check
   Fields9 bw0, bw1;          // batched nonlinear forward: the shots' levels, stacked per field
   int batchShots = 0;
+  AcqTable acqA, acqB;       // injected points of the running pass (a gradient's two propagations)
+  bool tailReady = false;    // the running pass's steps carry their surroundings in the launch (StepTail)
+  // the level the last step wrote, to be recorded by the next step's launch (or flushRecord)
+  struct Pending {
+    bool on = false;
+    float* outL = nullptr;   // slices its and its+1, or with `its` the whole array
+    float* outR = nullptr;
+    int its = 0, k = 0;
+  } pending;
+  // nonlinear propagation of a grid whose rows are no multiple of four cells: the same grid in rows
+  // rounded up, which the TMA stepper takes (its medium a copy of this context's)
+  Context* padded = nullptr;
+  bool paddedMedium = false;
   std::unordered_map<unsigned long long, CUtensorMap> tmaps;  // (pointer, box) -> tensor map
   std::vector<void*> owned;  // every device allocation of this context
   // working wavefields (primary propagation)
@@ -203,6 +226,7 @@ int createContext(const ContextDesc& d, Context** out) {
   GridConst& g = c->g;
   g.nz = d.nz; g.nx = d.nx; g.ny = d.ny; g.minPad = d.minPad;
   g.yOff = 0; g.nyTaper = d.ny;
+  g.pz = d.nz;
   g.freeSurface = d.freeSurface ? 1 : 0;
   g.yStride = (long long)d.nz * d.nx;
   g.n = g.yStride * d.ny;
@@ -258,6 +282,10 @@ void destroyContext(Context* c) {
     c->evPool.push_back(t.b);
   }
   for (cudaEvent_t e : c->evPool) cudaEventDestroy(e);
+  if (c->padded) {
+    c->padded->st = c->st;
+    destroyContext(c->padded);
+  }
   for (void* p : c->owned) cudaFreeAsync(p, c->st);
   c->owned.clear();
   if (c->st) cudaStreamSynchronize(c->st);
@@ -297,6 +325,7 @@ int setMedium(Context* c, const float* const* planes, bool onDevice) {
   c->ckptValid = false;
   c->tailValid = false;
   c->premCond = -1.0;
+  c->paddedMedium = false;
   return E3D_OK;
 }
 
@@ -438,7 +467,7 @@ static int tensorMap(Context* c, const float* ptr, int boxZ, int boxX, const CUt
   E3D_ARG((reinterpret_cast<unsigned long long>(ptr) & 15) == 0, "field not 16-byte aligned");
   CUtensorMap m;
   cuuint64_t dims[4] = {(cuuint64_t)c->d.nz, (cuuint64_t)c->d.nx, (cuuint64_t)c->d.ny, (cuuint64_t)std::max(shots, 1)};
-  cuuint64_t strides[3] = {(cuuint64_t)c->d.nz * 4, (cuuint64_t)c->g.yStride * 4, (cuuint64_t)c->g.n * 4};
+  cuuint64_t strides[3] = {(cuuint64_t)c->g.pz * 4, (cuuint64_t)c->g.yStride * 4, (cuuint64_t)c->g.n * 4};
   cuuint32_t box[4] = {(cuuint32_t)boxZ, (cuuint32_t)boxX, 1, 1};
   cuuint32_t es[4] = {1, 1, 1, 1};
   CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, shots > 0 ? 4 : 3, const_cast<float*>(ptr), dims, strides,
@@ -525,54 +554,182 @@ static int launchSplit(Context* c, const StepPtrs& p, int tiz, int tix, int nyi)
   const int yChunk = (nyi + chunks - 1) / chunks;
   chunks = (nyi + yChunk - 1) / yChunk;
   kStepSplit<MODE, STAGES, MINB><<<dim3(tiz, tix, 2 * chunks), dim3(TZ, 8), smem, c->st>>>(mp, p, c->g, yChunk,
-                                                                                              chunks, 1, 0);
+                                                                                              chunks);
   return E3D_OK;
 }
 
-// One step of `shots` shots stacked per field (fields of n*shots floats), 3-stage split stepper.
-template <int MODE>
-static int launchSplitBatch(Context* c, const StepPtrs& p, int shots) {
-  constexpr size_t smem = (size_t)3 * SPL_STAGE_F * sizeof(float);
-  static std::atomic<unsigned long long> configured{0};
-  E3D_RET(ensureSmemAttr((const void*)kStepSplit<MODE, 3, 3, true>, smem, configured));
-  SplitMaps mp;
-  E3D_RET(buildSplitMaps(c, p, mp, shots));
+// Launch shape of the paired stepper: z tiles, x tiles and y runs of yChunk planes per role.
+struct PairShape {
+  int tilesZ, tilesX, chunks, yChunk;
+};
+
+static PairShape pairShape(const Context* c, int shots) {
+  PairShape s;
   const GridConst& g = c->g;
-  const int tiz = (g.nz - 2 * FAT + TZ - 1) / TZ;
-  const int tix = (g.nx - 2 * FAT + 7) / 8;
+  s.tilesZ = (g.nz - 2 * FAT + TZ - 1) / TZ;
+  s.tilesX = (g.nx - 2 * FAT + 7) / 8;
   const int nyi = g.ny - 2 * FAT;
-  int chunks = c->yChunks > 0 ? std::min(c->yChunks, nyi) : (nyi + 31) / 32;
-  chunks = std::max(chunks, 1);
-  const int yChunk = (nyi + chunks - 1) / chunks;
-  chunks = (nyi + yChunk - 1) / yChunk;
-  kStepSplit<MODE, 3, 3, true><<<dim3(tiz * shots, tix, 2 * chunks), dim3(TZ, 8), smem, c->st>>>(
-      mp, p, c->g, yChunk, chunks, shots, g.n);
+  int chunks = c->yChunks > 0 ? std::min(c->yChunks, nyi) : 0;
+  if (!chunks) {
+    // The CTAs run in waves of three per SM and each pays about three planes of start-up (window
+    // loads, first copies): pick the y runs that minimise waves * (planes + 3).  Runs stay within 44
+    // planes: on large grids neighbouring tiles then stay close enough for their halos to meet in
+    // L2.  Measured on B200, bare steps, against runs of 32 planes: 72x72x60 cells 26.6 -> 10.3 us,
+    // 104x104x96 36.6 -> 24.8, 168x168x152 119.7 -> 104.9, 168x200x188 167.8 -> 150.2; from
+    // 296x296x288 on within the spread.
+    const long long tiles = 2LL * s.tilesZ * s.tilesX * std::max(shots, 1), slots = 3LL * c->numSMs;
+    long long best = -1;
+    for (int P = std::min(nyi, 44); P >= std::min(nyi, 2); P--) {
+      const int ch = (nyi + P - 1) / P;
+      const long long cost = (tiles * ch + slots - 1) / slots * (P + 3);
+      if (best < 0 || cost < best) {
+        best = cost;
+        chunks = ch;
+      }
+    }
+  }
+  s.yChunk = (nyi + chunks - 1) / chunks;
+  s.chunks = (nyi + s.yChunk - 1) / s.yChunk;
+  return s;
+}
+
+// The paired stepper takes every forward and time-reversed step that fuses no decimation.
+static bool pairPath(const Context* c, int mode, const StepPtrs& p) {
+  return c->loader == 8 && mode != STEP_ADJ_EXACT && c->g.pz % 4 == 0 && p.accL[0] == nullptr;
+}
+
+// Paired split stepper (two z cells per thread, blockDim TZ/2 x 8), with the injection and recording
+// of `tail`.  Plain launches: programmatic ones (the next step's CTAs waiting in freed slots) measured
+// slower on B200, 108.7 against 103.4 us a step at 168x152x171 cells and 12.3 against 10.5 at 72x72x60
+// with 8-plane runs, because the early CTAs take their slots unevenly.
+template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE>
+static int launchPair(Context* c, const StepPtrs& p, const StepTail& tail, int shots) {
+  constexpr size_t smem = (size_t)STAGES * SPL_STAGE_F * sizeof(float);
+  static std::atomic<unsigned long long> configured{0};
+  E3D_RET(ensureSmemAttr((const void*)kStepSplitPair<MODE, STAGES, MINB, BATCH, SS, EDGE>, smem, configured));
+  SplitMaps mp;
+  E3D_RET(buildSplitMaps(c, p, mp, BATCH ? shots : 0));
+  const PairShape s = pairShape(c, shots);
+  kStepSplitPair<MODE, STAGES, MINB, BATCH, SS, EDGE>
+      <<<dim3(s.tilesZ * shots, s.tilesX, 2 * s.chunks + tail.recBlocks), dim3(TZ / 2, 8), smem, c->st>>>(
+          mp, p, c->g, s.yChunk, s.chunks, shots, tail);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
 
-// Paired split stepper (two z cells per thread, blockDim TZ/2 x 8): the y runs of launchSplit.
-template <int MODE, int STAGES, int MINB>
-static int launchSplitPair(Context* c, const StepPtrs& p, int tiz, int tix, int nyi) {
-  constexpr size_t smem = (size_t)STAGES * SPL_STAGE_F * sizeof(float);
-  static std::atomic<unsigned long long> configured{0};
-  E3D_RET(ensureSmemAttr((const void*)kStepSplitPair<MODE, STAGES, MINB>, smem, configured));
-  SplitMaps mp;
-  E3D_RET(buildSplitMaps(c, p, mp));
-  int chunks = c->yChunks > 0 ? std::min(c->yChunks, nyi) : (nyi + 31) / 32;
-  chunks = std::max(chunks, 1);
-  const int yChunk = (nyi + chunks - 1) / chunks;
-  chunks = (nyi + yChunk - 1) / yChunk;
-  kStepSplitPair<MODE, STAGES, MINB><<<dim3(tiz, tix, 2 * chunks), dim3(TZ / 2, 8), smem, c->st>>>(mp, p, c->g,
-                                                                                                   yChunk, chunks);
+template <int MODE>
+static int launchPairVariant(Context* c, const StepPtrs& p, const StepTail& tail) {
+  if (tail.surface || c->g.nz % 2) return launchPair<MODE, 3, 3, false, false, true>(c, p, tail, 1);
+  if (c->stages == 4) return launchPair<MODE, 4, 2, false, false, false>(c, p, tail, 1);
+  if (c->stages == 2) return launchPair<MODE, 2, 4, false, false, false>(c, p, tail, 1);
+  return launchPair<MODE, 3, 3, false, false, false>(c, p, tail, 1);
+}
+
+// Bins the points of a device set by the CTAs that update them (shots > 1: stacked grids).
+static int buildAcq(Context* c, AcqTable& t, const DevSignals& set, bool skipNormal, int shots) {
+  t.n = set.off[NCOMP];
+  if (t.n == 0) return E3D_OK;
+  const PairShape s = pairShape(c, shots);
+  AcqBins b;
+  b.pos = set.pos;
+  for (int i = 0; i <= NCOMP; i++) b.off[i] = set.off[i];
+  b.tilesZ = s.tilesZ; b.tilesX = s.tilesX; b.chunks = s.chunks; b.yChunk = s.yChunk;
+  b.nshots = shots; b.skipNormal = skipNormal ? 1 : 0;
+  const int owners = s.tilesZ * shots * s.tilesX * 2 * s.chunks;
+  if (t.rowCap < (size_t)owners + 1) {
+    devFree(c, t.row);
+    devFree(c, t.cursor);
+    t.row = t.cursor = nullptr;
+    t.rowCap = 0;
+    E3D_RET(devAlloc(c, (void**)&t.row, ((size_t)owners + 1) * sizeof(int)));
+    E3D_RET(devAlloc(c, (void**)&t.cursor, ((size_t)owners + 1) * sizeof(int)));
+    t.rowCap = (size_t)owners + 1;
+  }
+  if (t.entryCap < (size_t)t.n) {
+    devFree(c, t.entries);
+    t.entries = nullptr;
+    t.entryCap = 0;
+    E3D_RET(devAlloc(c, (void**)&t.entries, (size_t)t.n * sizeof(AcqEntry)));
+    t.entryCap = (size_t)t.n;
+  }
+  E3D_CUDA_TRY(cudaMemsetAsync(t.cursor, 0, (size_t)owners * sizeof(int), c->st));
+  c->launches += 3;
+  kAcqCount<<<(t.n + 255) / 256, 256, 0, c->st>>>(b, c->g, t.cursor);
+  kAcqScan<<<1, 1024, 0, c->st>>>(t.cursor, t.row, owners);
+  kAcqFill<<<(t.n + 255) / 256, 256, 0, c->st>>>(b, c->g, t.cursor, t.entries);
+  E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
 
-template <int MODE>
-static int launchSplitPairVariant(Context* c, const StepPtrs& p, int tiz, int tix, int nyi) {
-  if (c->stages == 4) return launchSplitPair<MODE, 4, 2>(c, p, tiz, tix, nyi);
-  if (c->stages == 2) return launchSplitPair<MODE, 2, 4>(c, p, tiz, tix, nyi);
-  return launchSplitPair<MODE, 3, 3>(c, p, tiz, tix, nyi);
+// Sets of up to this many points are injected by the stepper's CTAs; larger ones by a launch of their
+// own.  Measured on B200: a shot's sources (24 points) cost nothing beside the step, where their
+// launch took 4 us a step; 1.6 M points (150 x 150 receivers, premultiplied) lengthened the step by 92
+// us against 52 us for the launch; 115 thousand by 8 us against 6.
+constexpr int kTailInjectMax = 8192;
+
+// Prepares the steps of a pass to inject `set` in the stepper launch (table t; t.n = 0 where they do
+// not: many points, or no memory for the table).
+static int prepareInject(Context* c, AcqTable& t, const DevSignals& set, bool premultiplied, int shots = 1) {
+  t.n = 0;
+  if (set.off[NCOMP] == 0 || set.off[NCOMP] > kTailInjectMax) return E3D_OK;
+  const int st = buildAcq(c, t, set, premultiplied, shots);
+  if (st != E3D_ERR_OOM) return st;
+  cudaGetLastError();
+  t.n = 0;
+  return E3D_OK;
+}
+
+// Injection half of a tail: slices sigL and sigR, or (idx) the array sig at the device index plus off.
+static void tailInject(const Context* c, const AcqTable& a, StepTail& t, const DevSignals& s, const float* sigL,
+                       const float* sigR, int k, const int* idx = nullptr, int off = 0, bool premultiplied = false) {
+  if (a.n == 0) return;
+  t.inRow = a.row;
+  t.in = a.entries;
+  t.sig = sigL;
+  t.sigR = sigR;
+  t.inL = c->filt[k];
+  t.inR = c->filt[c->hfilt + k];
+  t.its = idx;
+  t.inOff = off;
+  t.nIn = s.off[NCOMP];
+  t.prem = premultiplied ? 1 : 0;
+  for (int i = 0; i < 3; i++) t.offC[i] = s.off[SXX + i];
+}
+
+static SparseSet sparseSet(const DevSignals& s) {
+  SparseSet r;
+  r.pos = s.pos;
+  for (int i = 0; i <= NCOMP; i++) r.off[i] = s.off[i];
+  return r;
+}
+
+// Recording half: the pending level, which is this step's current one.
+static void tailRecord(Context* c, StepTail& t, const DevSignals& s, int shots, const int* idx = nullptr) {
+  Context::Pending& q = c->pending;
+  if (!q.on) return;
+  q.on = false;
+  t.out = sparseSet(s);
+  const long long per = (long long)(TZ / 2 * 8) * REC_PER_THREAD;
+  const PairShape p = pairShape(c, shots);
+  const long long layer = (long long)p.tilesZ * shots * p.tilesX;
+  t.recBlocks = (int)((((long long)s.off[NCOMP] + per - 1) / per + layer - 1) / layer);
+  t.rec = q.outL;
+  t.recR = q.outR;
+  t.outL = c->filt[q.k];
+  t.outR = c->filt[c->hfilt + q.k];
+  if (idx) t.its = idx;
+  t.outOff = q.its;
+}
+
+// Leaves the level the step just launched writes to be recorded (slices outL and outR, or the array
+// outL at coarse time its) with filter weights k.
+static void recordLater(Context* c, const DevSignals& s, float* outL, float* outR, int its, int k) {
+  if (s.off[NCOMP] == 0) return;
+  c->pending.on = true;
+  c->pending.outL = outL;
+  c->pending.outR = outR;
+  c->pending.its = its;
+  c->pending.k = k;
 }
 
 template <int MODE>
@@ -631,7 +788,7 @@ static int launchVariant(Context* c, const StepPtrs& p, dim3 grid, int yChunk) {
   }
 }
 
-static int launchStepRaw(Context* c, int mode, const StepPtrs& p);
+static int launchStepRaw(Context* c, int mode, const StepPtrs& p, const StepTail* tail);
 
 static cudaEvent_t takeEvent(Context* c) {
   if (c->evPool.empty()) {
@@ -671,12 +828,12 @@ struct TimedLaunch {
 };
 
 // Every stepper launch goes through here: counts it and samples its time.
-static int launchStep(Context* c, int mode, const StepPtrs& p) {
+static int launchStep(Context* c, int mode, const StepPtrs& p, const StepTail* tail = nullptr) {
   c->launches++;
   // launches that also fuse a decimation or a secondary source are kept apart (mode + 3)
   const bool fused = p.accL[0] != nullptr || p.ssL[0] != nullptr;
   TimedLaunch t(c, mode + (fused ? 3 : 0));
-  return launchStepRaw(c, mode, p);
+  return launchStepRaw(c, mode, p, tail);
 }
 
 int setKernelTiming(Context* c, int every) {
@@ -732,7 +889,7 @@ static int chooseChunks(const Context* c, long long tiles, int nyi, int perSM) {
   return chunks;
 }
 
-static int launchStepRaw(Context* c, int mode, const StepPtrs& p) {
+static int launchStepRaw(Context* c, int mode, const StepPtrs& p, const StepTail* tail) {
   const GridConst& g = c->g;
   const int tiz = (g.nz - 2 * FAT + TZ - 1) / TZ;
   const int tix = (g.nx - 2 * FAT + c->tx - 1) / c->tx;
@@ -744,15 +901,17 @@ static int launchStepRaw(Context* c, int mode, const StepPtrs& p) {
   // it keeps the long runs.
   int chunks = chooseChunks(c, tiles, nyi);
   const bool dual = mode == STEP_ADJ_EXACT && p.oP[0] != nullptr;
-  // the split stepper (loader 6; loader 7: all but the exact adjoint, which keeps kStepTma; loader
-  // 8: loader 7 with two z cells per thread) takes every step without a fused decimation or
-  // secondary source
-  if (c->loader == 8 && mode != STEP_ADJ_EXACT && g.nz % 4 == 0 && p.accL[0] == nullptr && p.ssL[0] == nullptr) {
-    const int tixS = (g.nx - 2 * FAT + 7) / 8;
-    if (mode == STEP_FWD) E3D_RET(launchSplitPairVariant<STEP_FWD>(c, p, tiz, tixS, nyi));
-    else E3D_RET(launchSplitPairVariant<STEP_ADJ_REVERSED>(c, p, tiz, tixS, nyi));
-    E3D_LAUNCH_CHECK();
-    return E3D_OK;
+  // the split stepper (loader 6; loader 7: all but the exact adjoint, which keeps kStepTma) takes
+  // every step without a fused decimation or secondary source; loader 8's paired form takes the
+  // secondary source of a forward step too
+  if (pairPath(c, mode, p)) {
+    const StepTail none{};
+    const StepTail& t = tail ? *tail : none;
+    if (p.ssL[0]) {
+      if (mode == STEP_FWD) return launchPair<STEP_FWD, 3, 3, false, true, false>(c, p, t, 1);
+    } else {
+      return mode == STEP_FWD ? launchPairVariant<STEP_FWD>(c, p, t) : launchPairVariant<STEP_ADJ_REVERSED>(c, p, t);
+    }
   }
   if ((c->loader == 6 || (c->loader == 7 && mode != STEP_ADJ_EXACT)) && g.nz % 4 == 0 && p.accL[0] == nullptr &&
       p.ssL[0] == nullptr) {
@@ -799,22 +958,21 @@ static int launchStepRaw(Context* c, int mode, const StepPtrs& p) {
 
 // Injection of time slices sigL (its) and sigR (its+1), filter weights k.
 static int launchInjectSlices(Context* c, const StepPtrs& p, const DevSignals& s, const float* sigL,
-                              const float* sigR, int k) {
-  SparseSet ss;
-  ss.pos = s.pos;
-  for (int i = 0; i <= NCOMP; i++) ss.off[i] = s.off[i];
+                              const float* sigR, int k, int surface = 0) {
+  const SparseSet ss = sparseSet(s);
   const int n = s.off[NCOMP];
   if (n == 0) return E3D_OK;
   c->launches++;
-  kInject<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss, sigL, sigR, c->filt[k], c->filt[c->hfilt + k]);
+  kInject<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss, sigL, sigR, c->filt[k], c->filt[c->hfilt + k], surface);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
 
 // Injection from a time-major [nts][ntot] signal array at coarse time its.
-static int launchInject(Context* c, const StepPtrs& p, const DevSignals& s, const float* sig, int its, int k) {
+static int launchInject(Context* c, const StepPtrs& p, const DevSignals& s, const float* sig, int its, int k,
+                        int surface = 0) {
   const size_t ntot = (size_t)s.off[NCOMP];
-  return launchInjectSlices(c, p, s, sig + (size_t)its * ntot, sig + (size_t)(its + 1) * ntot, k);
+  return launchInjectSlices(c, p, s, sig + (size_t)its * ntot, sig + (size_t)(its + 1) * ntot, k, surface);
 }
 
 static int launchRecordSlices(Context* c, const StepPtrs& p, const DevSignals& s, float* outL, float* outR, int k) {
@@ -824,7 +982,7 @@ static int launchRecordSlices(Context* c, const StepPtrs& p, const DevSignals& s
   const int n = s.off[NCOMP];
   if (n == 0) return E3D_OK;
   c->launches++;
-  kRecord<<<(n + 127) / 128, 128, 0, c->st>>>(p, ss, outL, outR, c->filt[k], c->filt[c->hfilt + k]);
+  kRecord<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss, outL, outR, c->filt[k], c->filt[c->hfilt + k]);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
@@ -832,6 +990,16 @@ static int launchRecordSlices(Context* c, const StepPtrs& p, const DevSignals& s
 static int launchRecord(Context* c, const StepPtrs& p, const DevSignals& s, float* out, int its, int k) {
   const size_t ntot = (size_t)s.off[NCOMP];
   return launchRecordSlices(c, p, s, out + (size_t)its * ntot, out + (size_t)(its + 1) * ntot, k);
+}
+
+// Records the pending level `lev` in a launch of its own (the end of a pass).
+static int flushRecord(Context* c, const Fields9& lev, const DevSignals& s, bool wholeArray) {
+  Context::Pending q = c->pending;
+  c->pending.on = false;
+  if (!q.on) return E3D_OK;
+  StepPtrs p{};
+  for (int k = 0; k < NCOMP; k++) p.o[k] = lev.p[k];
+  return wholeArray ? launchRecord(c, p, s, q.outL, q.its, q.k) : launchRecordSlices(c, p, s, q.outL, q.outR, q.k);
 }
 
 static int launchExtractSource(Context* c, const StepPtrs& p, const DevSignals& s, float* out, int its, int k) {
@@ -1060,14 +1228,15 @@ __global__ void kSetIndex(int* its, int v) {
 }
 
 static int launchInjectIdx(Context* c, const StepPtrs& p, const DevSignals& s, const float* sig, const int* idx,
-                           int k) {
+                           int off, int k, int surface = 0) {
   SparseSet ss;
   ss.pos = s.pos;
   for (int i = 0; i <= NCOMP; i++) ss.off[i] = s.off[i];
   const int n = s.off[NCOMP];
   if (n == 0) return E3D_OK;
   c->launches++;
-  kInjectIdx<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss, sig, idx, c->filt[k], c->filt[c->hfilt + k]);
+  kInjectIdx<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss, sig, idx, off, c->filt[k],
+                                                 c->filt[c->hfilt + k], surface);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
@@ -1079,16 +1248,19 @@ static int launchRecordIdx(Context* c, const StepPtrs& p, const DevSignals& s, f
   const int n = s.off[NCOMP];
   if (n == 0) return E3D_OK;
   c->launches++;
-  kRecordIdx<<<(n + 127) / 128, 128, 0, c->st>>>(p, ss, out, idx, c->filt[k], c->filt[c->hfilt + k]);
+  kRecordIdx<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss, out, idx, c->filt[k], c->filt[c->hfilt + k]);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
+
+// Whether the passes of this context can leave injection and recording to the stepper launch.
+static bool takesTail(const Context* c) { return c->loader == 8 && c->g.pz % 4 == 0; }
 
 // One coarse block of the nonlinear loops.  Forward (propElasticFwdGpu_3D):
 // per fine step it2 = 1..sub  step -> inject (k=it2-1) -> [free surface] ->
 // record (k=it2) -> swap.  Time-reversed (propElasticAdjGpu_3D, quirk Q7):
 // it2 = sub-1..0  step -> inject data (k=it2+1) -> [free surface] -> record
-// source (k=it2) -> swap.  With idx the coarse index is read on the device.
+// source (k=it2) -> swap.  With idx the coarse index is read on the device and its counts from there.
 // Fine step s of coarse block its (the reference's loop order): step, inject, free surface,
 // record; the new level ends in c->w1.
 static int nlSubStep(Context* c, bool adjoint, const DevSignals& srcSet, const DevSignals& recSet, float* srcSig,
@@ -1101,8 +1273,30 @@ static int nlSubStep(Context* c, bool adjoint, const DevSignals& srcSet, const D
   const int it2 = adjoint ? sub - 1 - s : s + 1;
   const int kIn = adjoint ? it2 + 1 : it2 - 1;
   StepPtrs p = makeStep(c, c->w0, c->w1);
-  E3D_RET(launchStep(c, adjoint ? STEP_ADJ_REVERSED : STEP_FWD, p));
-  if (idx) E3D_RET(launchInjectIdx(c, p, inSet, inSig, idx, kIn));
+  const int mode = adjoint ? STEP_ADJ_REVERSED : STEP_FWD;
+  if (c->tailReady) {
+    StepTail t{};
+    t.surface = c->g.freeSurface;
+    const size_t ni = (size_t)inSet.off[NCOMP];
+    if (idx) tailInject(c, c->acqA, t, inSet, inSig, nullptr, kIn, idx, its);
+    else tailInject(c, c->acqA, t, inSet, inSig + its * ni, inSig + (its + 1) * ni, kIn);
+    if (!idx && c->pending.on) {  // an absolute sample: the slices themselves
+      const size_t no = (size_t)outSet.off[NCOMP];
+      c->pending.outL = outSig + c->pending.its * no;
+      c->pending.outR = c->pending.outL + no;
+    }
+    tailRecord(c, t, outSet, 1, idx);
+    E3D_RET(launchStep(c, mode, p, &t));
+    if (c->acqA.n == 0) {
+      if (idx) E3D_RET(launchInjectIdx(c, p, inSet, inSig, idx, its, kIn, t.surface));
+      else E3D_RET(launchInject(c, p, inSet, inSig, its, kIn, t.surface));
+    }
+    recordLater(c, outSet, outSig, nullptr, its, it2);
+    swapF(c->w0, c->w1);
+    return E3D_OK;
+  }
+  E3D_RET(launchStep(c, mode, p));
+  if (idx) E3D_RET(launchInjectIdx(c, p, inSet, inSig, idx, 0, kIn));
   else E3D_RET(launchInject(c, p, inSet, inSig, its, kIn));
   E3D_RET(launchFreeSurface(c, p, adjoint ? -1.f : 1.f));
   if (idx) E3D_RET(launchRecordIdx(c, p, outSet, outSig, idx, it2));
@@ -1117,18 +1311,19 @@ static int nlBlock(Context* c, bool adjoint, const DevSignals& srcSet, const Dev
   return E3D_OK;
 }
 
-// Capture one coarse block (block(idx) with the device-resident coarse index,
-// then the index advanced by `delta`) into an executable graph.  Counted launches
-// of the capture are returned in *perBlock and taken back out of the context's count.
+// Capture `group` coarse blocks (block(u*delta, idx): the device-resident coarse index plus u*delta),
+// then the index advanced past them, into an executable graph.  Counted launches of the capture are
+// returned in *perGroup and taken back out of the context's count.
 template <class Block>
-static int captureBlockWith(Context* c, Block block, int delta, cudaGraphExec_t* exec, long long* perBlock) {
+static int captureBlocks(Context* c, Block block, int group, int delta, cudaGraphExec_t* exec, long long* perGroup) {
   const long long before = c->launches;
   cudaGraph_t graph = nullptr;
   E3D_CUDA_TRY(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
   c->inCapture = true;
-  int st = block(c->blockIndex);
+  int st = E3D_OK;
+  for (int u = 0; u < group && st == E3D_OK; u++) st = block(u * delta, c->blockIndex);
   if (st == E3D_OK) {
-    kAdvanceIndex<<<1, 32, 0, c->st>>>(c->blockIndex, delta);
+    kAdvanceIndex<<<1, 32, 0, c->st>>>(c->blockIndex, group * delta);
     c->launches++;
     if (cudaGetLastError() != cudaSuccess) {
       setLastError("index advance launch failed", __FILE__, __LINE__);
@@ -1137,7 +1332,7 @@ static int captureBlockWith(Context* c, Block block, int delta, cudaGraphExec_t*
   }
   c->inCapture = false;
   const cudaError_t e = cudaStreamEndCapture(c->st, &graph);
-  *perBlock = c->launches - before;
+  *perGroup = c->launches - before;
   c->launches = before;
   if (st == E3D_OK && e != cudaSuccess) {
     setLastError(cudaGetErrorString(e), __FILE__, __LINE__);
@@ -1154,36 +1349,49 @@ static int captureBlockWith(Context* c, Block block, int delta, cudaGraphExec_t*
   return st;
 }
 
-// Replay of coarse blocks 1..blocks-1 after block 0 ran eagerly: one captured block (two when
-// sub is odd, for the two pointer parities of the leapfrog levels lv0/lv1), the coarse index on
-// the device starting at `next` and moving by `delta`.
+// Coarse blocks 1..blocks-1 after block 0 ran eagerly, most of them as replays of a captured group
+// of blocks with the coarse index on the device; block(its, null) launches coarse block its itself,
+// next and delta are block 1's index and the way it moves.  Steps that inject and record in their own
+// launch take their sample relative to the index, so eight blocks make a group and the index moves
+// once per group (one launch of every 33 at sub = 4 instead of one of 5); the others read the index
+// as it stands, one block at a time, with two graphs for the two pointer parities of the leapfrog
+// levels lv0/lv1 when sub is odd.
 template <class Block>
 static int replayBlocks(Context* c, Block block, int blocks, int next, int delta, Fields9& lv0, Fields9& lv1) {
+  const int sub = c->d.sub, rest = blocks - 1;
+  int group = 1;
+  if (c->tailReady) {
+    group = std::min(rest, 8);
+    if (sub % 2) group &= ~1;  // whole swaps of the two levels
+  }
+  const int eager = group ? rest % group : rest;
+  for (int b = 0; b < eager; b++) E3D_RET(block(next + b * delta, nullptr));
+  if (eager == rest) return E3D_OK;
   if (!c->blockIndex) E3D_RET(devAlloc(c, (void**)&c->blockIndex, sizeof(int)));
-  kSetIndex<<<1, 32, 0, c->st>>>(c->blockIndex, next);
+  kSetIndex<<<1, 32, 0, c->st>>>(c->blockIndex, next + eager * delta);
   c->launches++;
   E3D_LAUNCH_CHECK();
-  const int sub = c->d.sub;
-  const int ng = (sub % 2) ? 2 : 1;
+  const int ng = (group * sub % 2) ? 2 : 1, runs = (rest - eager) / group;
   cudaGraphExec_t exec[2] = {nullptr, nullptr};
-  long long perBlock[2] = {0, 0};
+  long long perGroup[2] = {0, 0};
   int st = E3D_OK;
-  for (int i = 0; i < ng && st == E3D_OK; i++) st = captureBlockWith(c, block, delta, &exec[i], &perBlock[i]);
-  for (int b = 1; b < blocks && st == E3D_OK; b++) {
-    const int i = (b - 1) % ng;
-    const cudaError_t e = cudaGraphLaunch(exec[i], c->st);
+  c->pending.its = -delta;  // a replay's first step records the block before it
+  for (int i = 0; i < ng && st == E3D_OK; i++) {
+    st = captureBlocks(c, block, group, delta, &exec[i], &perGroup[i]);
+    c->pending.its = -delta;
+  }
+  c->pending.its = next + (rest - 1) * delta;
+  for (int b = 0; b < runs && st == E3D_OK; b++) {
+    const cudaError_t e = cudaGraphLaunch(exec[b % ng], c->st);
     if (e != cudaSuccess) {
       setLastError(cudaGetErrorString(e), __FILE__, __LINE__);
       st = E3D_ERR_CUDA;
     }
-    c->launches += perBlock[i];
+    c->launches += perGroup[b % ng];
   }
-  // the host-side level pointers follow the replayed blocks: each capture swapped them sub
-  // times, and capture ng - 1 more blocks' worth than ran
-  if (st == E3D_OK) {
-    const long long swapsCaptured = (long long)ng * sub, swapsRun = (long long)(blocks - 1) * sub;
-    if ((swapsCaptured + swapsRun) % 2) swapF(lv0, lv1);
-  }
+  // the host-side level pointers follow the replayed blocks: the captures swapped them ng * group *
+  // sub times, the replays stand for runs * group * sub swaps
+  if (st == E3D_OK && ((long long)(ng + runs) * group * sub) % 2) swapF(lv0, lv1);
   for (int i = 0; i < ng; i++)
     if (exec[i]) cudaGraphExecDestroy(exec[i]);
   return st;
@@ -1238,10 +1446,10 @@ int validateDeviceSets(Context* c, const DevSignals& a, const DevSignals& b, int
 // ---------------------------------------------------------------------------
 // Batched nonlinear forward: `shots` shots of one medium advanced together.
 // Each field holds the shots stacked (shot s at offset s*n), every fine step is
-// one split-stepper launch for all shots (CTAs of one tile for consecutive
-// shots adjacent, so the medium tile comes from L2 after the first shot), one
-// injection and one recording launch over the combined tables, whose
-// positions carry the shot offset.  Loop order of propElasticFwdGpu_3D.
+// one paired-stepper launch for all shots (CTAs of one tile for consecutive
+// shots adjacent, so the medium tile comes from L2 after the first shot), which
+// also injects and records over the combined tables, whose positions carry
+// the shot offset.  Loop order of propElasticFwdGpu_3D.
 // ---------------------------------------------------------------------------
 int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const DevSignals& recSet,
                          const float* srcSig, float* recSig) {
@@ -1270,19 +1478,32 @@ int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const 
   }
   const int nts = c->d.nts, sub = c->d.sub;
   E3D_CUDA_TRY(cudaMemsetAsync(recSig, 0, (size_t)std::max(recSet.off[NCOMP], 1) * nts * sizeof(float), c->st));
-  // one coarse block (its, or the device index idx) of all shots
+  E3D_RET(prepareInject(c, c->acqA, srcSet, false, shots));
+  c->tailReady = true;
+  c->pending = {};
+  // one coarse block (its, or its samples after the device index idx) of all shots
   auto block = [&](int its, const int* idx) -> int {
     for (int it2 = 1; it2 <= sub; it2++) {
       StepPtrs p = makeStep(c, c->bw0, c->bw1);
+      StepTail t{};
+      const size_t ns = (size_t)srcSet.off[NCOMP], nr = (size_t)recSet.off[NCOMP];
+      if (idx) tailInject(c, c->acqA, t, srcSet, srcSig, nullptr, it2 - 1, idx, its);
+      else tailInject(c, c->acqA, t, srcSet, srcSig + its * ns, srcSig + (its + 1) * ns, it2 - 1);
+      if (!idx && c->pending.on) {
+        c->pending.outL = recSig + c->pending.its * nr;
+        c->pending.outR = c->pending.outL + nr;
+      }
+      tailRecord(c, t, recSet, shots, idx);
       {
         c->launches++;
-        TimedLaunch t(c, STEP_FWD);
-        E3D_RET(launchSplitBatch<STEP_FWD>(c, p, shots));
+        TimedLaunch tl(c, STEP_FWD);
+        E3D_RET((launchPair<STEP_FWD, 3, 3, true, false, false>(c, p, t, shots)));
       }
-      if (idx) E3D_RET(launchInjectIdx(c, p, srcSet, srcSig, idx, it2 - 1));
-      else E3D_RET(launchInject(c, p, srcSet, srcSig, its, it2 - 1));
-      if (idx) E3D_RET(launchRecordIdx(c, p, recSet, recSig, idx, it2));
-      else E3D_RET(launchRecord(c, p, recSet, recSig, its, it2));
+      if (c->acqA.n == 0) {
+        if (idx) E3D_RET(launchInjectIdx(c, p, srcSet, srcSig, idx, its, it2 - 1));
+        else E3D_RET(launchInject(c, p, srcSet, srcSig, its, it2 - 1));
+      }
+      recordLater(c, recSet, recSig, nullptr, its, it2);
       swapF(c->bw0, c->bw1);
     }
     return E3D_OK;
@@ -1291,20 +1512,86 @@ int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const 
   const bool graph = c->graphLoop && c->st != nullptr && c->timingEvery == 0 && blocks >= 4;
   if (!graph) {
     for (int its = 0; its < blocks; its++) E3D_RET(block(its, nullptr));
+  } else {
+    // the time loop as replays of captured coarse blocks, as nlPropagateDevice
+    E3D_RET(block(0, nullptr));
+    E3D_RET(replayBlocks(c, block, blocks, 1, 1, c->bw0, c->bw1));
+  }
+  return flushRecord(c, c->bw1, recSet, true);
+}
+
+// The context of the same grid in rows of a multiple of four cells, with this context's medium; *out
+// null where the device has no memory for it (the grid then runs on the plain stepper).
+static int paddedContext(Context* c, Context** out) {
+  *out = nullptr;
+  Context* t = c->padded;
+  if (!t) {
+    t = new Context();
+    t->d = c->d;
+    t->g = c->g;
+    t->g.pz = (c->d.nz + 3) / 4 * 4;
+    t->g.yStride = (long long)t->g.pz * c->d.nx;
+    t->g.n = t->g.yStride * c->d.ny;
+    t->hfilt = c->hfilt;
+    t->filt = c->filt;
+    t->dtsInv = c->dtsInv;
+    t->numSMs = c->numSMs;
+    t->haveMedium = true;
+    c->padded = t;
+    c->paddedMedium = false;
+  }
+  t->st = c->st;
+  t->stages = c->stages;
+  t->yChunks = c->yChunks;
+  t->graphLoop = c->graphLoop;
+  t->timingEvery = c->timingEvery;
+  int st = E3D_OK;
+  for (int k = 0; k < NMED && st == E3D_OK; k++)
+    if (!t->med[k]) st = devAlloc(t, (void**)&t->med[k], (size_t)t->g.n * sizeof(float));
+  if (st == E3D_OK) st = allocFields(t, t->w0, false);
+  if (st == E3D_OK) st = allocFields(t, t->w1, false);
+  if (st == E3D_ERR_OOM) {
+    cudaGetLastError();
+    destroyContext(t);
+    c->padded = nullptr;
     return E3D_OK;
   }
-  // the time loop as replays of one captured coarse block, as nlPropagateDevice
-  E3D_RET(block(0, nullptr));
-  return replayBlocks(c, [&](const int* idx) { return block(0, idx); }, blocks, 1, 1, c->bw0, c->bw1);
+  E3D_RET(st);
+  if (!c->paddedMedium) {
+    for (int k = 0; k < NMED; k++)
+      E3D_CUDA_TRY(cudaMemcpy2DAsync(t->med[k], (size_t)t->g.pz * sizeof(float), c->med[k],
+                                     (size_t)c->d.nz * sizeof(float), (size_t)c->d.nz * sizeof(float),
+                                     (size_t)c->d.nx * c->d.ny, cudaMemcpyDeviceToDevice, c->st));
+    c->paddedMedium = true;
+  }
+  *out = t;
+  return E3D_OK;
 }
 
 int nlPropagateDevice(Context* c, bool adjoint, const DevSignals& srcSet, const DevSignals& recSet, float* srcSig,
                       float* recSig) {
   E3D_ARG(c && c->haveMedium, "medium not set");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
+  if (c->loader == 8 && c->g.pz % 4 != 0) {
+    // rows that no bulk copy can start on: the same grid in rounded-up rows.  Measured on B200 at
+    // 101 x 91 x 117 cells against the plain stepper: see kStepSplitPair
+    Context* t = nullptr;
+    E3D_RET(paddedContext(c, &t));
+    if (t) {
+      const long long before = t->launches;
+      const int st = nlPropagateDevice(t, adjoint, srcSet, recSet, srcSig, recSig);
+      c->launches += t->launches - before;
+      c->timed.insert(c->timed.end(), t->timed.begin(), t->timed.end());
+      t->timed.clear();
+      return st;
+    }
+  }
   E3D_RET(allocFields(c, c->w0, true));
   E3D_RET(allocFields(c, c->w1, true));
-  const int nts = c->d.nts, sub = c->d.sub;
+  c->tailReady = takesTail(c);
+  c->pending = {};
+  if (c->tailReady) E3D_RET(prepareInject(c, c->acqA, adjoint ? recSet : srcSet, false));
+  const int nts = c->d.nts;
   const int blocks = nts - 1;
   float* outSig = adjoint ? srcSig : recSig;
   const DevSignals& outSet = adjoint ? srcSet : recSet;
@@ -1314,12 +1601,13 @@ int nlPropagateDevice(Context* c, bool adjoint, const DevSignals& srcSet, const 
   const bool graph = c->graphLoop && c->st != nullptr && c->timingEvery == 0 && blocks >= 4;
   if (!graph) {
     for (int b = 0; b < blocks; b++) E3D_RET(nlBlock(c, adjoint, srcSet, recSet, srcSig, recSig, first + dir * b, nullptr));
-    return E3D_OK;
+  } else {
+    E3D_RET(nlBlock(c, adjoint, srcSet, recSet, srcSig, recSig, first, nullptr));
+    E3D_RET(replayBlocks(
+        c, [&](int its, const int* idx) { return nlBlock(c, adjoint, srcSet, recSet, srcSig, recSig, its, idx); },
+        blocks, first + dir, dir, c->w0, c->w1));
   }
-  E3D_RET(nlBlock(c, adjoint, srcSet, recSet, srcSig, recSig, first, nullptr));
-  return replayBlocks(
-      c, [&](const int* idx) { return nlBlock(c, adjoint, srcSet, recSet, srcSig, recSig, 0, idx); }, blocks,
-      first + dir, dir, c->w0, c->w1);
+  return flushRecord(c, c->w1, outSet, true);
 }
 
 int nlPropagateHost(Context* c, bool adjoint, float* const* model, float* const* data, const HostGeom& src,
@@ -1507,6 +1795,9 @@ int nlPropagateSlabsHost(Context* const* slabs, int nSlabs, int nyGlobal, bool a
     if (st == E3D_OK) st = adjoint ? stageSignalsIn(c, r.R, in) : stageSignalsZero(c, r.R);
     if (st == E3D_OK) st = allocFields(c, c->w0, true);
     if (st == E3D_OK) st = allocFields(c, c->w1, true);
+    c->tailReady = takesTail(c);
+    c->pending = {};
+    if (st == E3D_OK && c->tailReady) st = prepareInject(c, c->acqA, adjoint ? r.R.set : r.S.set, false);
     if (st == E3D_OK) cu(cudaEventCreateWithFlags(&r.stepped, cudaEventDisableTiming));
     if (st == E3D_OK) cu(cudaEventCreateWithFlags(&r.copied, cudaEventDisableTiming));
   }
@@ -1559,6 +1850,7 @@ int nlPropagateSlabsHost(Context* const* slabs, int nSlabs, int nyGlobal, bool a
       r.sig[outSide][k].assign(std::max<size_t>(r.rows[outSide][k].size(), 1) * nts, 0.f);
       out[k] = r.sig[outSide][k].data();
     }
+    if (st == E3D_OK) st = flushRecord(c, c->w1, adjoint ? r.S.set : r.R.set, true);
     if (st == E3D_OK) st = stageSignalsOut(c, adjoint ? r.S : r.R, out);
     if (st == E3D_OK) st = checkPipeError(c);  // synchronizes the slab's stream
     if (st == E3D_OK)
@@ -1938,22 +2230,36 @@ static int ensurePert(Context* c) {
 // scattered propagation so that S[t] (needs V[t-1..t+1]) is ready when the
 // scattered block t-1 starts.  Four velocity slots and two secondary-source
 // slots rotate; nothing leaves the device.
+static int sourceBlockRing(Context* c, long long& m, int its, const DevSignals& srcSet, const float* srcSig,
+                           float* vLeft, int leftMode, float* vRight);
+
 static int bornForwardDevice(Context* c, const DevSignals& srcSet, const DevSignals& recSet, const float* srcSig,
                              float* recSig) {
   const int nts = c->d.nts, sub = c->d.sub;
-  E3D_RET(allocFields(c, c->s0, true));
-  E3D_RET(allocFields(c, c->s1, true));
+  // with a ring of source levels one launch per block decimates them and the steps carry no
+  // accumulators (188 -> 140 B per cell and step)
+  const bool ring = ringLevels(c) > 0;
+  if (ring) {
+    E3D_RET(ensureRing(c, c->srcRing, c->s0, c->s1, ringLevels(c)));
+  } else {
+    E3D_RET(allocFields(c, c->s0, true));
+    E3D_RET(allocFields(c, c->s1, true));
+  }
+  c->tailReady = takesTail(c);
+  c->pending = {};
+  if (c->tailReady) E3D_RET(prepareInject(c, c->acqA, srcSet, false));
   E3D_RET(allocFields(c, c->w0, true));
   E3D_RET(allocFields(c, c->w1, true));
   E3D_RET(allocFields(c, c->ss[0], true));
   E3D_RET(allocFields(c, c->ss[1], true));
   E3D_RET(ensureVSlots(c, 4));
   c->tailValid = false;  // the rotating slots overwrite a kept source segment
-  for (int i = 0; i < 4; i++)
+  for (int i = 0; i < 4 && !ring; i++)
     E3D_CUDA_TRY(cudaMemsetAsync(c->vSlots[i], 0, (size_t)3 * c->g.n * sizeof(float), c->st));
   E3D_CUDA_TRY(cudaMemsetAsync(recSig, 0, (size_t)std::max(recSet.off[NCOMP], 1) * nts * sizeof(float), c->st));
   auto V = [&](int t) -> float* { return (t < 0 || t >= nts) ? nullptr : c->vSlots[t % 4]; };
   auto SS = [&](int t) -> Fields9& { return c->ss[t % 2]; };
+  long long m = 0;      // source ring level
   int nextS = 0;        // next secondary source to compute
   int nextScatter = 0;  // next scattered block
   auto scatterBlock = [&](int its) -> int {
@@ -1965,17 +2271,30 @@ static int bornForwardDevice(Context* c, const DevSignals& srcSet, const DevSign
       }
       p.ssWl = c->filt[it2 - 1];
       p.ssWr = c->filt[c->hfilt + it2 - 1];
-      E3D_RET(launchStep(c, STEP_FWD, p));
-      E3D_RET(launchRecord(c, p, recSet, recSig, its, it2));
+      if (c->tailReady) {
+        StepTail t{};
+        float* ol = recSig + (size_t)its * recSet.off[NCOMP];
+        tailRecord(c, t, recSet, 1);
+        E3D_RET(launchStep(c, STEP_FWD, p, &t));
+        recordLater(c, recSet, ol, ol + recSet.off[NCOMP], its, it2);
+      } else {
+        E3D_RET(launchStep(c, STEP_FWD, p));
+        E3D_RET(launchRecord(c, p, recSet, recSig, its, it2));
+      }
       swapF(c->w0, c->w1);
     }
     return E3D_OK;
   };
   auto computeS = [&](int t) -> int { return launchImaging(c, false, t, V(t - 1), V(t), V(t + 1), SS(t)); };
   for (int b = 0; b < nts - 1; b++) {
-    // slot of V[b+1] was last used by V[b-3]; clear it before accumulating
-    E3D_CUDA_TRY(cudaMemsetAsync(V(b + 1), 0, (size_t)3 * c->g.n * sizeof(float), c->st));
-    E3D_RET(sourceBlock(c, b, srcSet, srcSig, V(b), V(b + 1)));
+    if (ring) {
+      // block b adds its left part to V[b] and writes V[b+1]'s first part over V[b-3]
+      E3D_RET(sourceBlockRing(c, m, b, srcSet, srcSig, V(b), b == 0 ? 2 : 1, V(b + 1)));
+    } else {
+      // slot of V[b+1] was last used by V[b-3]; clear it before accumulating
+      E3D_CUDA_TRY(cudaMemsetAsync(V(b + 1), 0, (size_t)3 * c->g.n * sizeof(float), c->st));
+      E3D_RET(sourceBlock(c, b, srcSet, srcSig, V(b), V(b + 1)));
+    }
     // V[b] is complete: S[b-1] can be formed
     while (nextS <= b - 1) E3D_RET(computeS(nextS++));
     while (nextScatter + 1 < nextS) E3D_RET(scatterBlock(nextScatter++));
@@ -1987,7 +2306,7 @@ static int bornForwardDevice(Context* c, const DevSignals& srcSet, const DevSign
     while (nextScatter + 1 < nextS && nextScatter < nts - 1) E3D_RET(scatterBlock(nextScatter++));
   }
   while (nextScatter < nts - 1) E3D_RET(scatterBlock(nextScatter++));
-  return E3D_OK;
+  return flushRecord(c, c->w1, recSet, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -2467,8 +2786,12 @@ static int sourceBlockRing(Context* c, long long& m, int its, const DevSignals& 
   auto S = [&](long long k) -> Fields9& { return ringAt(c->srcRing, k); };
   for (int it2 = 1; it2 <= c->d.sub; it2++) {
     StepPtrs p = makeRingStep(c, S(m - 1), S(m), S(m + 1));
-    E3D_RET(launchStep(c, STEP_FWD, p));
-    E3D_RET(launchInject(c, afterStep(p), srcSet, srcSig, its, it2 - 1));
+    StepTail t{};
+    const float* sl = srcSig + (size_t)its * srcSet.off[NCOMP];
+    const bool inside = c->tailReady && c->acqA.n > 0;
+    if (inside) tailInject(c, c->acqA, t, srcSet, sl, sl + srcSet.off[NCOMP], it2 - 1);
+    E3D_RET(launchStep(c, STEP_FWD, p, &t));
+    if (!inside) E3D_RET(launchInject(c, afterStep(p), srcSet, srcSig, its, it2 - 1));
     m++;
   }
   if ((vLeft && leftMode) || vRight) E3D_RET(launchDecimate(c, m, vLeft, leftMode, vRight));
@@ -2488,6 +2811,9 @@ static int sourcePassRing(Context* c, const DevSignals& srcSet, const DevSignals
     bool prem = false;  // known before the plan, which then leaves out the dual state's levels
     E3D_RET(premultipliedAdjoint(c, prem));
   }
+  c->tailReady = takesTail(c);
+  c->pending = {};
+  if (c->tailReady) E3D_RET(prepareInject(c, c->acqA, srcSet, false));
   E3D_RET(prepareCheckpoints(c, L, nseg));
   const int nts = c->d.nts, sub = c->d.sub, blocks = nts - 1;
   const size_t nr = recSet ? (size_t)recSet->off[NCOMP] : 0;
@@ -2509,6 +2835,12 @@ static int sourcePassRing(Context* c, const DevSignals& srcSet, const DevSignals
     return vc ? c->vSlots[(t - tailBeg) % 2] : c->vSlots[t - tailBeg];
   };
   auto S = [&](long long k) -> Fields9& { return ringAt(c->srcRing, k); };
+  // slice b of the trace ring is complete: to the irregular receivers, and its slot cleared for slice b+2
+  auto sliceDone = [&](int b) -> int {
+    E3D_RET(traceGather(c, *map, (int)nr, ring + (b % 2) * nr, recSig + (size_t)b * rows));
+    if (nr) E3D_CUDA_TRY(cudaMemsetAsync(ring + (b % 2) * nr, 0, nr * sizeof(float), c->st));
+    return E3D_OK;
+  };
   long long m = 0;  // levels -1 and 0 are the zero initial state
   int nextCk = 1;
   for (int b = 0; b < blocks; b++) {
@@ -2519,6 +2851,20 @@ static int sourcePassRing(Context* c, const DevSignals& srcSet, const DevSignals
     }
     for (int it2 = 1; it2 <= sub; it2++) {
       StepPtrs p = makeRingStep(c, S(m - 1), S(m), S(m + 1));
+      if (c->tailReady) {
+        StepTail t{};
+        const float* sl = srcSig + (size_t)b * srcSet.off[NCOMP];
+        if (c->acqA.n) tailInject(c, c->acqA, t, srcSet, sl, sl + srcSet.off[NCOMP], it2 - 1);
+        if (recSig) tailRecord(c, t, *recSet, 1);
+        E3D_RET(launchStep(c, STEP_FWD, p, &t));
+        if (!c->acqA.n) E3D_RET(launchInject(c, afterStep(p), srcSet, srcSig, b, it2 - 1));
+        if (ring) recordLater(c, *recSet, ring + (b % 2) * nr, ring + ((b + 1) % 2) * nr, b, it2);
+        else if (recSig) recordLater(c, *recSet, recSig + b * nr, recSig + (b + 1) * nr, b, it2);
+        // this launch recorded the last level of block b-1: its slice is complete
+        if (ring && it2 == 1 && b > 0) E3D_RET(sliceDone(b - 1));
+        m++;
+        continue;
+      }
       E3D_RET(launchStep(c, STEP_FWD, p));
       const StepPtrs q = afterStep(p);
       E3D_RET(launchInject(c, q, srcSet, srcSig, b, it2 - 1));
@@ -2532,11 +2878,11 @@ static int sourcePassRing(Context* c, const DevSignals& srcSet, const DevSignals
       // V[b] is complete: store it; its slot next receives V[b+2], written by block b+1
       E3D_RET(packVelocity(c, A(b), c->vStore[b - tailBeg]));
     }
-    if (ring) {
-      // slice b is complete; its ring slot is reused for slice b+2
-      E3D_RET(traceGather(c, *map, (int)nr, ring + (b % 2) * nr, recSig + (size_t)b * rows));
-      if (nr) E3D_CUDA_TRY(cudaMemsetAsync(ring + (b % 2) * nr, 0, nr * sizeof(float), c->st));
-    }
+    if (ring && !c->tailReady) E3D_RET(sliceDone(b));
+  }
+  if (c->tailReady && recSig) {
+    E3D_RET(flushRecord(c, S(m), *recSet, false));
+    if (ring) E3D_RET(sliceDone(blocks - 1));
   }
   // V[nts-1] has no block of its own: complete after block nts-2
   if (vc) E3D_RET(packVelocity(c, A(nts - 1), c->vStore[nts - 1 - tailBeg]));
@@ -2607,6 +2953,12 @@ static int adjointPassRing(Context* c, const DevSignals& srcSet, const DevSignal
     return vc ? c->vSlots[(t - winStart) % 2] : c->vSlots[t - winStart];
   };
   auto W = [&](long long k) -> Fields9& { return ringAt(c->adjRing, k); };
+  // the recomputed source steps inject in their launch, and so do premultiplied steps of few receivers
+  c->tailReady = takesTail(c);
+  c->pending = {};
+  c->acqB.n = 0;
+  if (c->tailReady) E3D_RET(prepareInject(c, c->acqA, srcSet, false));
+  if (c->tailReady && prem) E3D_RET(prepareInject(c, c->acqB, recSet, true));
   long long ma = 0;  // adjoint levels -1 and 0: the zero final state
   const bool tailKept = c->tailValid;
   if (nseg > 1) c->tailValid = false;
@@ -2659,6 +3011,13 @@ static int adjointPassRing(Context* c, const DevSignals& srcSet, const DevSignal
         // a_new = G (G a_old - D(P_cur)), P_new = M a_new reads
         // P_new = G (G P_old - M D(P_cur)) with M applied term by term: the
         // time-reversed stepper (stepAdjGpu_3D's update) on P.
+        if (prem && c->acqB.n) {
+          StepTail t{};
+          tailInject(c, c->acqB, t, recSet, dataSlice(its), dataSlice(its + 1), it2 + 1, nullptr, 0, true);
+          E3D_RET(launchStep(c, STEP_ADJ_REVERSED, p, &t));
+          ma++;
+          continue;
+        }
         E3D_RET(launchStep(c, prem ? STEP_ADJ_REVERSED : STEP_ADJ_EXACT, p));
         const StepPtrs q = afterStep(p);
         if (prem) E3D_RET(launchInjectPremultiplied(c, q, recSet, dataSlice(its), dataSlice(its + 1), it2 + 1));
@@ -2887,6 +3246,7 @@ int nlPropagateStatic(const ContextDesc& d, const float* const* planes, bool adj
   GridConst g{};
   g.nz = d.nz; g.nx = d.nx; g.ny = d.ny; g.minPad = d.minPad;
   g.yOff = 0; g.nyTaper = d.ny;
+  g.pz = d.nz;
   g.yStride = (long long)d.nz * d.nx;
   g.n = n;
   const double kc[4] = {1.196289062541883, -0.079752604188901, 0.009570312506634, -6.975446437140719e-04};
@@ -2969,11 +3329,11 @@ int nlPropagateStatic(const ContextDesc& d, const float* const* planes, bool adj
         E3D_LAUNCH_CHECK();
         if (nS) {
           kInject<<<(nS + 127) / 128, 128, 0, st>>>(p, g, S, srcSig + its * ns, srcSig + (its + 1) * ns,
-                                                   filt[it2 - 1], filt[hfilt + it2 - 1]);
+                                                   filt[it2 - 1], filt[hfilt + it2 - 1], 0);
           E3D_LAUNCH_CHECK();
         }
         if (nR) {
-          kRecord<<<(nR + 127) / 128, 128, 0, st>>>(p, R, recSig + its * nr, recSig + (its + 1) * nr, filt[it2],
+          kRecord<<<(nR + 127) / 128, 128, 0, st>>>(p, g, R, recSig + its * nr, recSig + (its + 1) * nr, filt[it2],
                                                    filt[hfilt + it2]);
           E3D_LAUNCH_CHECK();
         }
@@ -2988,11 +3348,11 @@ int nlPropagateStatic(const ContextDesc& d, const float* const* planes, bool adj
         E3D_LAUNCH_CHECK();
         if (nR) {
           kInject<<<(nR + 127) / 128, 128, 0, st>>>(p, g, R, recSig + its * nr, recSig + (its + 1) * nr,
-                                                   filt[it2 + 1], filt[hfilt + it2 + 1]);
+                                                   filt[it2 + 1], filt[hfilt + it2 + 1], 0);
           E3D_LAUNCH_CHECK();
         }
         if (nS) {
-          kRecord<<<(nS + 127) / 128, 128, 0, st>>>(p, S, srcSig + its * ns, srcSig + (its + 1) * ns, filt[it2],
+          kRecord<<<(nS + 127) / 128, 128, 0, st>>>(p, g, S, srcSig + its * ns, srcSig + (its + 1) * ns, filt[it2],
                                                    filt[hfilt + it2]);
           E3D_LAUNCH_CHECK();
         }

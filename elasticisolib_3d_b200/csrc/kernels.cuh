@@ -47,6 +47,11 @@ struct SparseSet {
   int off[NCOMP + 1];
 };
 
+// Cell of a position given in unpadded rows (stacked shots carry shot * nz*nx*ny).
+__device__ __forceinline__ long long cellIndex(const GridConst& g, long long pos) {
+  return g.pz == g.nz ? pos : pos / g.nz * g.pz + pos % g.nz;
+}
+
 // Medium-premultiplied wavefield at one cell (stepAdjGpuBorn_3D, kernelsElaGpu_3D.cu:864-920).
 __device__ __forceinline__ void premultiply(const float* v, float rhox, float rhoy, float rhoz, float l2m, float lam,
                                             float muxz, float muxy, float muyz, float* q) {
@@ -723,20 +728,14 @@ __device__ __forceinline__ void splitIssuePlane(const CUtensorMap* mp, float* st
     tmaLoad3d(st + R::MED_OFF + k * SPL_INT_F, &mp[R::NH + 3 + R::NO + k], z0, x0, y, bar);
 }
 
-template <int MODE, bool ROLE_S, int STAGES, bool BATCH>
+template <int MODE, bool ROLE_S, int STAGES>
 __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs& p, const GridConst& g, int yChunk,
-                                          int chunk, float* smem, unsigned long long* bars, int nshots,
-                                          long long shotStride) {
+                                          int chunk, float* smem, unsigned long long* bars) {
   using R = SplitRole<ROLE_S>;
   constexpr int TXS = 8;
   const int tz = threadIdx.x, tx = threadIdx.y;
   const int tid = tx * TZ + tz;
-  // stacked shots: consecutive CTAs take one tile for consecutive shots, so a
-  // medium tile fetched for one shot is in L2 for the others
-  const int shot = BATCH ? (int)(blockIdx.x % nshots) : 0;
-  const int tileZ = BATCH ? (int)(blockIdx.x / nshots) : (int)blockIdx.x;
-  const long long soff = BATCH ? (long long)shot * shotStride : 0;
-  const int z0 = FAT + tileZ * TZ, x0 = FAT + blockIdx.y * TXS;
+  const int z0 = FAT + blockIdx.x * TZ, x0 = FAT + blockIdx.y * TXS;
   const int iz = z0 + tz, ix = x0 + tx;
   const bool active = (iz < g.nz - FAT) && (ix < g.nx - FAT);
   const int yBeg = FAT + chunk * yChunk;
@@ -751,7 +750,7 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
   if (tid == 0) {
     for (int s = 0; s < STAGES - 1; s++)
       if (yBeg + s < yEnd)
-        splitIssuePlane<ROLE_S, BATCH>(mp, smem + s * SPL_STAGE_F, &bars[s], yBeg + s, z0, x0, shot);
+        splitIssuePlane<ROLE_S, false>(mp, smem + s * SPL_STAGE_F, &bars[s], yBeg + s, z0, x0, 0);
   }
   float w[3][8];
   if (active) {
@@ -759,7 +758,7 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
     for (int q = 0; q < 3; q++)
 #pragma unroll
       for (int k = 0; k < 7; k++)
-        w[q][k] = __ldg(p.c[R::lead(q)] + soff + (long long)(yBeg + R::base(q) + k) * ys + col);
+        w[q][k] = __ldg(p.c[R::lead(q)] + (long long)(yBeg + R::base(q) + k) * ys + col);
   }
   const int dzx = min(min(topDistance(g, iz), ix - FAT), min(g.nz - iz - 1 - FAT, g.nx - ix - 1 - FAT));
   const float Gzx = (active && dzx < g.minPad) ? __ldg(g.taper + dzx) : 1.0f;
@@ -785,12 +784,11 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
       const int yn = y + STAGES - 1;
       int ns = slot + STAGES - 1;
       if (ns >= STAGES) ns -= STAGES;
-      if (yn < yEnd) splitIssuePlane<ROLE_S, BATCH>(mp, smem + ns * SPL_STAGE_F, &bars[ns], yn, z0, x0, shot);
+      if (yn < yEnd) splitIssuePlane<ROLE_S, false>(mp, smem + ns * SPL_STAGE_F, &bars[ns], yn, z0, x0, 0);
     }
     const float* st = smem + slot * SPL_STAGE_F;
     if (active) {
       const long long ic = (long long)y * ys + col;
-      const long long icf = ic + soff;  // this shot's cell in the stacked fields
 #pragma unroll
       for (int q = 0; q < 3; q++) w[q][7] = st[R::LEAD_OFF + q * SPL_INT_F + li];
       const float* cz = g.cz;
@@ -821,11 +819,11 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
 #pragma unroll
         for (int k = 0; k < 3; k++) nv[k] = G * (G * ov[k * SPL_INT_F] + up[k]);
 #pragma unroll
-        for (int k = 0; k < 3; k++) dst[VX + k][icf] = nv[k];
+        for (int k = 0; k < 3; k++) dst[VX + k][ic] = nv[k];
         if (MODE == STEP_ADJ_EXACT && p.oP[0]) {
-          p.oP[VX][icf] = nv[0] * rhox;
-          p.oP[VY][icf] = nv[1] * rhoy;
-          p.oP[VZ][icf] = nv[2] * rhoz;
+          p.oP[VX][ic] = nv[0] * rhox;
+          p.oP[VY][ic] = nv[1] * rhoy;
+          p.oP[VZ][ic] = nv[2] * rhoz;
         }
       } else {
         const float* tVX = st;
@@ -855,14 +853,14 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
 #pragma unroll
         for (int k = 0; k < 6; k++) nv[k] = G * (G * ov[k * SPL_INT_F] + up[k]);
 #pragma unroll
-        for (int k = 0; k < 6; k++) dst[SXX + k][icf] = nv[k];
+        for (int k = 0; k < 6; k++) dst[SXX + k][ic] = nv[k];
         if (MODE == STEP_ADJ_EXACT && p.oP[0]) {
-          p.oP[SXX][icf] = nv[0] * l2m + (nv[1] + nv[2]) * lam;
-          p.oP[SYY][icf] = nv[1] * l2m + (nv[0] + nv[2]) * lam;
-          p.oP[SZZ][icf] = nv[2] * l2m + (nv[0] + nv[1]) * lam;
-          p.oP[SXZ][icf] = nv[3] * muxz;
-          p.oP[SXY][icf] = nv[4] * muxy;
-          p.oP[SYZ][icf] = nv[5] * muyz;
+          p.oP[SXX][ic] = nv[0] * l2m + (nv[1] + nv[2]) * lam;
+          p.oP[SYY][ic] = nv[1] * l2m + (nv[0] + nv[2]) * lam;
+          p.oP[SZZ][ic] = nv[2] * l2m + (nv[0] + nv[1]) * lam;
+          p.oP[SXZ][ic] = nv[3] * muxz;
+          p.oP[SXY][ic] = nv[4] * muxy;
+          p.oP[SYZ][ic] = nv[5] * muyz;
         }
       }
 #pragma unroll
@@ -882,7 +880,9 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
 // instead of 16 single ones, an x derivative 8 instead of 16, and the old level,
 // medium and y-window planes one paired load per field; the new level is
 // stored as float2.  Each cell's arithmetic is kStepSplit's, term by term.
-// blockDim (TZ/2, 8); forward and time-reversed modes.
+// blockDim (TZ/2, 8); forward and time-reversed modes.  The launch also does
+// what surrounds the step: the free surface's images, a Born secondary source,
+// the injection of few points and the recording of the level before (StepTail).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float2 lds2(const float* t, int i) { return *reinterpret_cast<const float2*>(t + i); }
 
@@ -911,22 +911,196 @@ __device__ __forceinline__ void dMinusX2(const float* t, int i, int s, const flo
   r1 = c[0] * (p0.y - m1.y) + c[1] * (p1.y - m2.y) + c[2] * (p2.y - m3.y) + c[3] * (p3.y - m4.y);
 }
 
-template <int MODE, bool ROLE_S, int STAGES>
+// What a paired stepper launch does beside the step itself.
+//   Injection of few points (a shot's sources): every cell of a component is updated by one CTA of the
+//   launch (its role, y run and z/x tile), so that CTA can also inject into the points among its cells
+//   once its planes are stored, without a hazard between CTAs.  A table lists the points by owner
+//   (inRow[cta] .. inRow[cta + 1]); a kernel bins the positions once per call.
+//   Recording of the level before: the receivers of level n are read by the launch that advances
+//   level n to n+1, which only reads it, in CTAs of their own behind the stepper's (blockIdx.z beyond
+//   both roles), where they fill the last wave.
+struct AcqEntry {
+  unsigned long long cellComp;  // cell in the (stacked) fields, component in the top byte
+  float taper;                  // the sponge at the cell
+  int j;                        // column of the signal slices
+};
+constexpr int ACQ_COMP_SHIFT = 56;
+
+struct StepTail {
+  const int* inRow;       // injected points by owner (null: none)
+  const AcqEntry* in;
+  const float* sig;       // signal array (its given) or slice its; slice its+1 in sigR
+  const float* sigR;
+  float inL, inR;         // time-filter weights of the two slices
+  int prem;               // 1: the increments enter premultiplied by the medium (kInjectPremultiplied)
+  int offC[3];            // prem: first column of sxx, syy, szz
+  SparseSet out;          // recorded points of the current level (out.pos null: none)
+  int recBlocks;          // blockIdx.z layers of recording CTAs
+  float* rec;             // recorded array (its given) or slice its; slice its+1 in recR
+  float* recR;
+  float outL, outR;
+  const int* its;         // coarse time index on the device (replayed graphs), null: slices given
+  int inOff, outOff;      // coarse samples of the injection and the recording after it
+  long long nIn;          // columns per injected slice
+  int surface;            // 1: free-surface conditions on the new level (kFreeSurface's), injection included
+};
+
+__device__ __forceinline__ AcqEntry acqEntry(const AcqEntry* p) {
+  const uint4 w = __ldg(reinterpret_cast<const uint4*>(p));
+  AcqEntry e;
+  e.cellComp = (unsigned long long)w.y << 32 | w.x;
+  e.taper = __uint_as_float(w.z);
+  e.j = (int)w.w;
+  return e;
+}
+
+// One injected point.  fetch() loads what the injection reads (the increment, the field there and,
+// for premultiplied levels, the medium; an sxx entry of those stands for the three normal stresses),
+// apply() stores, so that several points of a thread are in flight.
+template <bool ROLE_S>
+struct AcqPoint {
+  static constexpr int N = ROLE_S ? 3 : 1;
+  int k;
+  long long i;
+  bool normal;
+  float a[N], f[N], m[2];
+
+  __device__ __forceinline__ void fetch(const StepTail& t, const AcqEntry& e, float l, float r, const float* sl,
+                                        const float* sr, float* const* dst, const float* const* med) {
+    k = (int)(e.cellComp >> ACQ_COMP_SHIFT);
+    i = (long long)(e.cellComp & ((1ULL << ACQ_COMP_SHIFT) - 1));
+    normal = ROLE_S && t.prem && k == SXX;
+    a[0] = e.taper * (l * t.inL + r * t.inR);
+    f[0] = __ldcg(dst[k] + i);
+    if (normal) {
+      const int row = e.j - t.offC[0];
+#pragma unroll
+      for (int c = 1; c < N; c++) {
+        a[c] = e.taper * (__ldg(sl + t.offC[c] + row) * t.inL + __ldg(sr + t.offC[c] + row) * t.inR);
+        f[c] = __ldcg(dst[SXX + c] + i);
+      }
+      m[0] = __ldg(med[L2M] + i);
+      m[1] = __ldg(med[LAM] + i);
+    } else if (t.prem) {
+      m[0] = __ldg(med[k < SXX ? k : k == SXZ ? MUXZ : k == SXY ? MUXY : MUYZ] + i);
+    }
+  }
+  __device__ __forceinline__ void apply(const StepTail& t, const GridConst& g, float* const* dst) const {
+    if (normal) {
+#pragma unroll
+      for (int c = 0; c < N; c++) {
+        const float o = c == 0 ? a[N / 2] + a[N - 1] : c == 1 ? a[0] + a[N - 1] : a[0] + a[N / 2];
+        dst[SXX + c][i] = f[c] + (a[c] * m[0] + o * m[1]);
+      }
+      return;
+    }
+    if (t.prem) {
+      dst[k][i] = f[0] + a[0] * m[0];
+      return;
+    }
+    const float v = f[0] + a[0];
+    if (t.surface) {
+      // the surface conditions hold after the injection: rows fixed by them take none, and a
+      // row with an image above the surface updates it
+      const int iz = (int)(i % g.pz);
+      if (iz == FAT && (k == VZ || k >= SZZ) && k != SXY) return;
+      if (k == SZZ && iz <= 2 * FAT) dst[k][i - 2 * (iz - FAT)] = -v;
+      if ((k == SXZ || k == SYZ) && iz <= 2 * FAT + 1) dst[k][i + (2 * FAT + 1 - 2 * iz)] = -v;
+    }
+    dst[k][i] = v;
+  }
+};
+
+// Injection into a CTA's own points i0..i1, after its last plane is stored.  Not inlined: in the
+// stepper's body its registers and code slowed the march of every CTA (measured on B200, steps without
+// points: 9.9 against 8.8 us at 72x72x60 cells), while few CTAs own points.
+template <bool ROLE_S, int NT>
+__device__ __noinline__ void stepInject(const StepTail& t, const GridConst& g, float* const* dst,
+                                        const float* const* med, int tid, int i0, int i1) {
+  constexpr int U = 4;  // points of a thread in flight
+  const long long n = t.nIn;
+  const float* sl = t.its ? t.sig + (__ldg(t.its) + t.inOff) * n : t.sig;
+  const float* sr = t.its ? sl + n : t.sigR;
+  __syncthreads();  // the CTA's stores are visible to its threads
+  for (int e = i0 + tid; e < i1; e += U * NT) {
+    AcqEntry en[U];
+    AcqPoint<ROLE_S> q[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) en[u] = acqEntry(t.in + min(e + u * NT, i1 - 1));
+#pragma unroll
+    for (int u = 0; u < U; u++) q[u].fetch(t, en[u], __ldg(sl + en[u].j), __ldg(sr + en[u].j), sl, sr, dst, med);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (e + u * NT < i1) q[u].apply(t, g, dst);
+  }
+}
+
+// Recording of the current level by CTA number `block` of the recording ones.
+constexpr int REC_PER_THREAD = 4;
+template <int NT>
+__device__ __forceinline__ void stepRecord(const StepTail& t, const GridConst& g, const float* const* cur, int block,
+                                           int tid) {
+  const int n = t.out.off[NCOMP];
+  const long long it = t.its ? __ldg(t.its) + t.outOff : 0;
+  float* ol = t.its ? t.rec + it * n : t.rec;
+  float* orr = t.its ? ol + n : t.recR;
+  const int j0 = block * (NT * REC_PER_THREAD) + tid;
+  float v[REC_PER_THREAD], l[REC_PER_THREAD], r[REC_PER_THREAD];
+#pragma unroll
+  for (int u = 0; u < REC_PER_THREAD; u++) {
+    const int j = j0 + u * NT;
+    if (j < n) {
+      int k = 0;
+#pragma unroll
+      for (int c = 1; c < NCOMP; c++) k += (j >= t.out.off[c]);
+      v[u] = __ldg(cur[k] + cellIndex(g, __ldg(t.out.pos + j)));
+      l[u] = ol[j];
+      r[u] = orr[j];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < REC_PER_THREAD; u++) {
+    const int j = j0 + u * NT;
+    if (j < n) {
+      ol[j] = l[u] + v[u] * t.outL;
+      orr[j] = r[u] + v[u] * t.outR;
+    }
+  }
+}
+
+// SS: a Born secondary source is added before the sponge (ssL, ssR weighted by ssWl, ssWr).
+// BATCH: nshots shots stacked per field (shot s at offset s*n), 4D field maps, blockIdx.x = tile *
+// nshots + shot: consecutive CTAs take one tile for consecutive shots, so a medium tile fetched for
+// one shot is in L2 for the others.
+// EDGE: rows of an odd number of cells or a free surface (tail.surface); the common form carries
+// neither's branches (measured on B200 at 72x72x60 cells, 4-plane runs: 8.9 against 9.5 us a step).
+template <int MODE, bool ROLE_S, int STAGES, bool BATCH, bool SS, bool EDGE>
 __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepPtrs& p, const GridConst& g,
-                                              int yChunk, int chunk, float* smem, unsigned long long* bars) {
+                                              int yChunk, int chunk, float* smem, unsigned long long* bars,
+                                              int nshots, const StepTail& tail) {
   static_assert(MODE != STEP_ADJ_EXACT, "the paired split stepper takes the forward and time-reversed modes");
   using R = SplitRole<ROLE_S>;
   constexpr int TXS = 8;
+  constexpr int NT = TZ / 2 * TXS;
   const int tz2 = threadIdx.x, tx = threadIdx.y;
   const int tid = tx * (TZ / 2) + tz2;
-  const int z0 = FAT + blockIdx.x * TZ, x0 = FAT + blockIdx.y * TXS;
+  const int shot = BATCH ? (int)(blockIdx.x % nshots) : 0;
+  const int tileZ = BATCH ? (int)(blockIdx.x / nshots) : (int)blockIdx.x;
+  const long long soff = BATCH ? (long long)shot * g.n : 0;
+  const int z0 = FAT + tileZ * TZ, x0 = FAT + blockIdx.y * TXS;
   const int iz = z0 + 2 * tz2, ix = x0 + tx;  // cells iz and iz+1
-  // nz - FAT is even (nz % 4 == 0) and iz is even, so both cells are inside or both outside
   const bool active = (iz < g.nz - FAT) && (ix < g.nx - FAT);
+  const bool pair = !EDGE || iz + 1 < g.nz - FAT;  // false for the last cell of an odd row
   const int yBeg = FAT + chunk * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz + soff;
+  const int cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  int i0 = 0, i1 = 0;  // this CTA's injected points
+  if (tail.inRow) {
+    i0 = __ldg(tail.inRow + cta);
+    i1 = __ldg(tail.inRow + cta + 1);
+  }
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) mbarInit(&bars[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -934,7 +1108,8 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
   __syncthreads();
   if (tid == 0) {
     for (int s = 0; s < STAGES - 1; s++)
-      if (yBeg + s < yEnd) splitIssuePlane<ROLE_S, false>(mp, smem + s * SPL_STAGE_F, &bars[s], yBeg + s, z0, x0, 0);
+      if (yBeg + s < yEnd)
+        splitIssuePlane<ROLE_S, BATCH>(mp, smem + s * SPL_STAGE_F, &bars[s], yBeg + s, z0, x0, shot);
   }
   float w0[3][8], w1[3][8];  // y-windows of cells iz and iz+1
   if (active) {
@@ -952,16 +1127,28 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     dzx[h] = min(min(topDistance(g, iz + h), ix - FAT), min(g.nz - iz - h - 1 - FAT, g.nx - ix - 1 - FAT));
-    Gzx[h] = (active && dzx[h] < g.minPad) ? __ldg(g.taper + dzx[h]) : 1.0f;
+    Gzx[h] = (active && (h == 0 || pair) && dzx[h] < g.minPad) ? __ldg(g.taper + dzx[h]) : 1.0f;
   }
   const int lc = (tx + HALO) * SZ + (2 * tz2 + HALO);
   const int li = tx * TZ + 2 * tz2;
   float* const* dst = p.nw[0] ? p.nw : p.o;
+  float* out[R::NO];  // this thread's column of the new level, held in registers over the march
+#pragma unroll
+  for (int k = 0; k < R::NO; k++) out[k] = (p.nw[0] ? p.nw[R::C0 + k] : p.o[R::C0 + k]) + col;
   int slot = 0;
   unsigned parity = 0;
   for (int y = yBeg; y < yEnd; y++) {
     const int dyy = yDistance(g, y);
     const float Gy = dyy < g.minPad ? __ldg(g.taper + dyy) : 1.0f;
+    const long long iy = (long long)y * ys;
+    float2 sL[SS ? R::NO : 1], sR[SS ? R::NO : 1];
+    if (SS && active) {
+#pragma unroll
+      for (int k = 0; k < R::NO; k++) {
+        sL[k] = __ldg(reinterpret_cast<const float2*>(p.ssL[R::C0 + k] + col + iy));
+        sR[k] = __ldg(reinterpret_cast<const float2*>(p.ssR[R::C0 + k] + col + iy));
+      }
+    }
     const bool ok = mbarWaitBounded(&bars[slot], (parity >> slot) & 1u);
     if (__syncthreads_or(!ok)) {
       if (tid == 0) {
@@ -976,11 +1163,10 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
       const int yn = y + STAGES - 1;
       int ns = slot + STAGES - 1;
       if (ns >= STAGES) ns -= STAGES;
-      if (yn < yEnd) splitIssuePlane<ROLE_S, false>(mp, smem + ns * SPL_STAGE_F, &bars[ns], yn, z0, x0, 0);
+      if (yn < yEnd) splitIssuePlane<ROLE_S, BATCH>(mp, smem + ns * SPL_STAGE_F, &bars[ns], yn, z0, x0, shot);
     }
     const float* st = smem + slot * SPL_STAGE_F;
     if (active) {
-      const long long ic = (long long)y * ys + col;
 #pragma unroll
       for (int q = 0; q < 3; q++) {
         const float2 v = lds2(st, R::LEAD_OFF + q * SPL_INT_F + li);
@@ -992,6 +1178,7 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
       const float* cy = g.cy;
       const float G[2] = {dyy < dzx[0] ? Gy : Gzx[0], dyy < dzx[1] ? Gy : Gzx[1]};
       const float sgn = (MODE == STEP_FWD) ? 1.0f : -1.0f;
+      float2 nv[R::NO];
       if (!ROLE_S) {
         const float* tSXX = st;
         const float* tSXY = st + SPL_HALO_F;
@@ -1016,11 +1203,15 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
         for (int k = 0; k < 3; k++) {
           const float2 rho = lds2(st, R::MED_OFF + k * SPL_INT_F + li);
           const float2 ov = lds2(st, R::OLD_OFF + k * SPL_INT_F + li);
-          float2 nv;
-          nv.x = G[0] * (G[0] * ov.x + sgn * (rho.x * fv[k][0]));
-          nv.y = G[1] * (G[1] * ov.y + sgn * (rho.y * fv[k][1]));
-          *reinterpret_cast<float2*>(dst[VX + k] + ic) = nv;
+          float ux = G[0] * ov.x + sgn * (rho.x * fv[k][0]);
+          float uy = G[1] * ov.y + sgn * (rho.y * fv[k][1]);
+          if (SS) {
+            ux += sL[k].x * p.ssWl + sR[k].x * p.ssWr;
+            uy += sL[k].y * p.ssWl + sR[k].y * p.ssWr;
+          }
+          nv[k] = make_float2(G[0] * ux, G[1] * uy);
         }
+        if (EDGE && tail.surface && iz == FAT) nv[VZ].x = 0.0f;  // the ghost row half a cell above the surface
       } else {
         const float* tVX = st;
         const float* tVY = st + SPL_HALO_F;
@@ -1059,11 +1250,40 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
 #pragma unroll
         for (int k = 0; k < 6; k++) {
           const float2 ov = lds2(st, R::OLD_OFF + k * SPL_INT_F + li);
-          float2 nv;
-          nv.x = G[0] * (G[0] * ov.x + up[k][0]);
-          nv.y = G[1] * (G[1] * ov.y + up[k][1]);
-          *reinterpret_cast<float2*>(dst[SXX + k] + ic) = nv;
+          float ux = G[0] * ov.x + up[k][0];
+          float uy = G[1] * ov.y + up[k][1];
+          if (SS) {
+            ux += sL[k].x * p.ssWl + sR[k].x * p.ssWr;
+            uy += sL[k].y * p.ssWl + sR[k].y * p.ssWr;
+          }
+          nv[k] = make_float2(G[0] * ux, G[1] * uy);
         }
+        if (EDGE && tail.surface && iz <= 2 * FAT) {
+          // stress imaging about the surface row FAT (the conditions kFreeSurface states), each row
+          // writing its image: szz rows FAT+1..2 FAT, sxz and syz rows FAT+1..2 FAT+1
+          if (iz == FAT) {
+            const float corr = sgn * G[0] * (-LAM_[0] * dzz[0] - (LAM_[0] * LAM_[0] / L2M_[0]) * (dxx[0] + dyy_[0]));
+            nv[0].x += corr;
+            nv[1].x += corr;
+            nv[2].x = 0.0f;
+            nv[3].x = -nv[3].y;
+            nv[5].x = -nv[5].y;
+            out[2][iy - 1] = -nv[2].y;
+          } else {
+            const int up2 = 2 * (iz - FAT);
+            out[2][iy - up2] = -nv[2].x;
+            if (iz < 2 * FAT) out[2][iy - up2 - 1] = -nv[2].y;
+            out[3][iy - up2 + 1] = -nv[3].x;
+            out[3][iy - up2] = -nv[3].y;
+            out[5][iy - up2 + 1] = -nv[5].x;
+            out[5][iy - up2] = -nv[5].y;
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < R::NO; k++) {
+        if (pair) *reinterpret_cast<float2*>(out[k] + iy) = nv[k];
+        else out[k][iy] = nv[k].x;
       }
 #pragma unroll
       for (int q = 0; q < 3; q++)
@@ -1075,29 +1295,96 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
     }
     slot = (slot + 1 == STAGES) ? 0 : slot + 1;
   }
+  if (i0 < i1) stepInject<ROLE_S, NT>(tail, g, dst, p.m, tid, i0, i1);
 }
 
-template <int MODE, int STAGES, int MINB>
-__global__ void __launch_bounds__(TZ / 2 * 8, MINB) kStepSplitPair(const __grid_constant__ SplitMaps mp, StepPtrs p,
-                                                                   GridConst g, int yChunk, int chunksV) {
-  extern __shared__ __align__(1024) float smem[];
-  __shared__ __align__(8) unsigned long long bars[STAGES];
-  if ((int)blockIdx.z < chunksV) splitRolePair<MODE, false, STAGES>(mp.v, p, g, yChunk, blockIdx.z, smem, bars);
-  else splitRolePair<MODE, true, STAGES>(mp.s, p, g, yChunk, blockIdx.z - chunksV, smem, bars);
-}
-
-// BATCH: nshots shots stacked per field (shot s at offset s * shotStride), field
-// maps 4D, blockIdx.x = tile * nshots + shot; forward and time-reversed modes only.
-template <int MODE, int STAGES, int MINB, bool BATCH = false>
-__global__ void __launch_bounds__(TZ * 8, MINB) kStepSplit(const __grid_constant__ SplitMaps mp, StepPtrs p,
-                                                            GridConst g, int yChunk, int chunksV, int nshots,
-                                                            long long shotStride) {
+template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE>
+__global__ void __launch_bounds__(TZ / 2 * 8, MINB) kStepSplitPair(const __grid_constant__ SplitMaps mp,
+                                                                   const __grid_constant__ StepPtrs p,
+                                                                   const __grid_constant__ GridConst g, int yChunk,
+                                                                   int chunksV, int nshots,
+                                                                   const __grid_constant__ StepTail tail) {
   extern __shared__ __align__(1024) float smem[];
   __shared__ __align__(8) unsigned long long bars[STAGES];
   if ((int)blockIdx.z < chunksV)
-    splitRole<MODE, false, STAGES, BATCH>(mp.v, p, g, yChunk, blockIdx.z, smem, bars, nshots, shotStride);
+    splitRolePair<MODE, false, STAGES, BATCH, SS, EDGE>(mp.v, p, g, yChunk, blockIdx.z, smem, bars, nshots, tail);
+  else if ((int)blockIdx.z >= 2 * chunksV)
+    stepRecord<TZ / 2 * 8>(tail, g, p.c, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * (blockIdx.z - 2 * chunksV)),
+                           threadIdx.y * (TZ / 2) + threadIdx.x);
   else
-    splitRole<MODE, true, STAGES, BATCH>(mp.s, p, g, yChunk, blockIdx.z - chunksV, smem, bars, nshots, shotStride);
+    splitRolePair<MODE, true, STAGES, BATCH, SS, EDGE>(mp.s, p, g, yChunk, blockIdx.z - chunksV, smem, bars, nshots, tail);
+}
+
+// Owner tables of the acquisition points (AcqEntry): the CTA that updates the component at the cell.
+// Launch shape of the paired stepper: z tiles (times shots), x tiles, y runs of yChunk planes, role V
+// before role S.  skipNormal: syy and szz entries are left out (premultiplied injection).
+struct AcqBins {
+  const long long* pos;  // positions in unpadded rows of nz (stacked shots carry shot * nz*nx*ny)
+  int off[NCOMP + 1];
+  int tilesZ, tilesX, chunks, yChunk, nshots, skipNormal;
+};
+__device__ __forceinline__ bool acqOwner(const AcqBins& b, const GridConst& g, int j, int* cta, AcqEntry* e) {
+  int k = 0;
+#pragma unroll
+  for (int c = 1; c < NCOMP; c++) k += (j >= b.off[c]);
+  if (b.skipNormal && (k == SYY || k == SZZ)) return false;
+  const long long p = b.pos[j];
+  const int iz = (int)(p % g.nz);
+  const long long row = p / g.nz;
+  const int ix = (int)(row % g.nx);
+  const long long pl = row / g.nx;
+  const int iy = (int)(pl % g.ny), shot = (int)(pl / g.ny);
+  const int tz = (iz - FAT) / TZ, tx = (ix - FAT) / 8, ch = (iy - FAT) / b.yChunk + (k >= SXX ? b.chunks : 0);
+  *cta = tz * b.nshots + shot + b.tilesZ * b.nshots * (tx + b.tilesX * ch);
+  if (e) {
+    const unsigned long long cell = (unsigned long long)(shot * g.n + (long long)iy * g.yStride + (long long)ix * g.pz + iz);
+    e->cellComp = cell | ((unsigned long long)k << ACQ_COMP_SHIFT);
+    e->taper = taperAt(g, iz, ix, iy);
+    e->j = j;
+  }
+  return true;
+}
+__global__ void kAcqCount(AcqBins b, GridConst g, int* count) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  int cta;
+  if (j < b.off[NCOMP] && acqOwner(b, g, j, &cta, nullptr)) atomicAdd(count + cta, 1);
+}
+// count[0..n) to exclusive sums row[0..n], one block; count is left holding the sums (the fill cursors)
+__global__ void __launch_bounds__(1024) kAcqScan(int* count, int* row, int n) {
+  __shared__ int part[1024];
+  const int per = (n + 1023) / 1024, b = threadIdx.x * per, e = min(b + per, n);
+  int s = 0;
+  for (int i = b; i < e; i++) s += count[i];
+  part[threadIdx.x] = s;
+  __syncthreads();
+  for (int o = 1; o < 1024; o <<= 1) {
+    const int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
+    __syncthreads();
+    part[threadIdx.x] += v;
+    __syncthreads();
+  }
+  int a = part[threadIdx.x] - s;
+  for (int i = b; i < e; i++) {
+    const int c = count[i];
+    count[i] = row[i] = a;
+    a += c;
+  }
+  if (threadIdx.x == 1023) row[n] = part[1023];
+}
+__global__ void kAcqFill(AcqBins b, GridConst g, int* cursor, AcqEntry* out) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  int cta;
+  AcqEntry e;
+  if (j < b.off[NCOMP] && acqOwner(b, g, j, &cta, &e)) out[atomicAdd(cursor + cta, 1)] = e;
+}
+
+template <int MODE, int STAGES, int MINB>
+__global__ void __launch_bounds__(TZ * 8, MINB) kStepSplit(const __grid_constant__ SplitMaps mp, StepPtrs p,
+                                                            GridConst g, int yChunk, int chunksV) {
+  extern __shared__ __align__(1024) float smem[];
+  __shared__ __align__(8) unsigned long long bars[STAGES];
+  if ((int)blockIdx.z < chunksV) splitRole<MODE, false, STAGES>(mp.v, p, g, yChunk, blockIdx.z, smem, bars);
+  else splitRole<MODE, true, STAGES>(mp.s, p, g, yChunk, blockIdx.z - chunksV, smem, bars);
 }
 
 // Recompute the premultiplied level at injected points (dual-state mode 2):
@@ -1454,7 +1741,7 @@ __global__ void __launch_bounds__(TZ * TX, MINB) kStepTma2(const __grid_constant
 // (ker_inject_source_* / ker_inject_data_*, kernelsElaGpu_3D.cu:11-52; the
 // source enters before the sponge, hence the taper at the point.)
 __device__ __forceinline__ void injectAt(const StepPtrs& p, const GridConst& g, const SparseSet& s,
-                                         const float* sigL, const float* sigR, float wl, float wr) {
+                                         const float* sigL, const float* sigR, float wl, float wr, int surface) {
   const int ntot = s.off[NCOMP];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ntot) return;
@@ -1465,13 +1752,22 @@ __device__ __forceinline__ void injectAt(const StepPtrs& p, const GridConst& g, 
   const float v = sigL[j] * wl + sigR[j] * wr;
   const int iz = (int)(pos % g.nz);
   const int ix = (int)((pos / g.nz) % g.nx);
-  const int iy = (int)((pos / g.yStride) % g.ny);  // positions of stacked shots carry shot * n
+  const int iy = (int)((pos / ((long long)g.nz * g.nx)) % g.ny);  // positions of stacked shots carry shot * n
   const float add = taperAt(g, iz, ix, iy) * v;
-  p.o[k][pos] += add;
+  const long long i = cellIndex(g, pos);
+  if (surface) {  // the step applied the surface conditions: as AcqPoint::apply
+    if (iz == FAT && (k == VZ || k >= SZZ) && k != SXY) return;
+    const float w = p.o[k][i] + add;
+    if (k == SZZ && iz <= 2 * FAT) p.o[k][i - 2 * (iz - FAT)] = -w;
+    if ((k == SXZ || k == SYZ) && iz <= 2 * FAT + 1) p.o[k][i + (2 * FAT + 1 - 2 * iz)] = -w;
+    p.o[k][i] = w;
+    return;
+  }
+  p.o[k][i] += add;
   // keep a decimation that the stepper fused in consistent with the injected value
   if (p.accL[0] != nullptr && k < p.nAcc) {
-    p.accL[k][pos] += add * p.accWl;
-    if (p.accR[0] != nullptr) p.accR[k][pos] += add * p.accWr;
+    p.accL[k][i] += add * p.accWl;
+    if (p.accR[0] != nullptr) p.accR[k][i] += add * p.accWr;
   }
 }
 
@@ -1502,16 +1798,16 @@ __global__ void kWriteTaper(TaperArg t, float* out) {
 }
 
 __global__ void kInject(StepPtrs p, GridConst g, SparseSet s, const float* sigL, const float* sigR, float wl,
-                        float wr) {
-  injectAt(p, g, s, sigL, sigR, wl, wr);
+                        float wr, int surface) {
+  injectAt(p, g, s, sigL, sigR, wl, wr, surface);
 }
 
 // The same with the coarse time index read on the device (time-major signals
-// [nts][ntot], slices its and its+1): the form a replayed CUDA graph uses.
-__global__ void kInjectIdx(StepPtrs p, GridConst g, SparseSet s, const float* sig, const int* its, float wl,
-                           float wr) {
-  const long long t = *its, ntot = s.off[NCOMP];
-  injectAt(p, g, s, sig + t * ntot, sig + (t + 1) * ntot, wl, wr);
+// [nts][ntot], slices *its + off and the next): the form a replayed CUDA graph uses.
+__global__ void kInjectIdx(StepPtrs p, GridConst g, SparseSet s, const float* sig, const int* its, int off, float wl,
+                           float wr, int surface) {
+  const long long t = *its + off, ntot = s.off[NCOMP];
+  injectAt(p, g, s, sig + t * ntot, sig + (t + 1) * ntot, wl, wr, surface);
 }
 
 // Advance the device-side coarse time index of a replayed coarse block.
@@ -1567,21 +1863,21 @@ __global__ void kFreeSurface(StepPtrs p, GridConst g, float sgn) {
 
 // outL[j] += field[pos]*wl; outR[j] += field[pos]*wr, with outL/outR the
 // time slices its and its+1 (ker_record_*, kernelsElaGpu_3D.cu:61-104)
-__device__ __forceinline__ void recordAt(const StepPtrs& p, const SparseSet& s, float* outL, float* outR, float wl,
-                                         float wr) {
+__device__ __forceinline__ void recordAt(const StepPtrs& p, const GridConst& g, const SparseSet& s, float* outL,
+                                         float* outR, float wl, float wr) {
   const int ntot = s.off[NCOMP];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ntot) return;
   int k = 0;
 #pragma unroll
   for (int c = 1; c < NCOMP; c++) k += (j >= s.off[c]);
-  const float v = p.o[k][s.pos[j]];
+  const float v = p.o[k][cellIndex(g, s.pos[j])];
   outL[j] += v * wl;
   outR[j] += v * wr;
 }
 
-__global__ void kRecord(StepPtrs p, SparseSet s, float* outL, float* outR, float wl, float wr) {
-  recordAt(p, s, outL, outR, wl, wr);
+__global__ void kRecord(StepPtrs p, GridConst g, SparseSet s, float* outL, float* outR, float wl, float wr) {
+  recordAt(p, g, s, outL, outR, wl, wr);
 }
 
 // Transpose of kInject: outL[j] += G(pos)*field[pos]*wl, outR[j] += G(pos)*field[pos]*wr, the
@@ -1602,9 +1898,9 @@ __global__ void kExtractSource(StepPtrs p, GridConst g, SparseSet s, float* outL
   outR[j] += v * wr;
 }
 
-__global__ void kRecordIdx(StepPtrs p, SparseSet s, float* out, const int* its, float wl, float wr) {
+__global__ void kRecordIdx(StepPtrs p, GridConst g, SparseSet s, float* out, const int* its, float wl, float wr) {
   const long long t = *its, ntot = s.off[NCOMP];
-  recordAt(p, s, out + t * ntot, out + (t + 1) * ntot, wl, wr);
+  recordAt(p, g, s, out + t * ntot, out + (t + 1) * ntot, wl, wr);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,0 +1,55 @@
+"""GPU: the paired stepper's launches over the sizes where they can go wrong, against the FP64 oracle.
+
+The default stepper injects few points and records in its own launch, applies the free surface there,
+and runs grids whose rows are no multiple of four cells in padded rows.  The cases cover rows of every
+remainder mod 4, odd axes, y runs down to two planes, an odd number of fine steps per sample, sources
+and receivers on both sides of the in-launch injection limit (8192 points over the nine components),
+records shorter and longer than a replayed group of eight samples, with and without the surface.
+The bound is the parity tests' 1e-5 relative L2 (FP32 rounding over the steps).
+"""
+import numpy as np
+import pytest
+
+from cases import random_signals, rel_l2
+from elasticisolib_3d_b200 import synthetic as S
+from elasticisolib_3d_b200.engine import Propagator
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+GRIDS = [(17, 13, 10, 12, 2, 3, 40), (29, 21, 19, 8, 3, 3, 60), (42, 24, 30, 21, 4, 1000, 50),
+         (30, 27, 18, 5, 5, 2, 950), (72, 40, 57, 6, 4, 4, 1000)]
+
+
+def _points(rng, nz, nx, ny, n):
+    cells = (nz - 8) * (nx - 8) * (ny - 8)
+    c = rng.permutation(cells)[:min(n, cells)]
+    z, x, y = c % (nz - 8) + 4, c // (nz - 8) % (nx - 8) + 4, c // ((nz - 8) * (nx - 8)) + 4
+    return ((y * nx + x) * nz + z).astype(np.int64)
+
+
+@pytest.mark.parametrize("surface", [0, 1])
+@pytest.mark.parametrize("adjoint", [False, True])
+@pytest.mark.parametrize("nz,nx,ny,nts,sub,nsrc,nrec", GRIDS)
+def test_paired_step_matches_oracle(nz, nx, ny, nts, sub, nsrc, nrec, adjoint, surface):
+    rng = np.random.default_rng(nz + 2 * surface)
+    el = S.elastic_from_velocity(*S.gaussian_perturbed_model((ny, nx, nz), 2500.0, 1443.0, 2000.0, 0.1, 2.0, 5))
+    dts = 0.0005 * sub
+    med = O.medium_planes(el, dts / sub, np.float32)
+    p = O.PropParams(nz, nx, ny, nts, sub, 3, 10.0, 10.0, 10.0, dts, free_surface=surface)
+    spos = [_points(rng, nz, nx, ny, nsrc) for _ in range(7)]
+    rpos = [_points(rng, nz, nx, ny, nrec) for _ in range(7)]
+    pr = Propagator(nz, nx, ny, nts, sub, 3, 10.0, 10.0, 10.0, dts, free_surface=surface)
+    pr.set_medium(med)
+    med64 = med.astype(np.float64)
+    for _ in range(2):  # a second call reuses the first one's tables and levels
+        sig = random_signals(rpos if adjoint else spos, nts, rng)
+        sig64 = [s.astype(np.float64) for s in sig]
+        if adjoint:
+            got = pr.nl_adjoint(sig, spos, rpos)
+            ref = O.nl_adjoint_reg(p, med64, sig64, spos, rpos, np.float64)
+        else:
+            got = pr.nl_forward(sig, spos, rpos)
+            ref = O.nl_forward_reg(p, med64, sig64, spos, rpos, np.float64)
+        assert rel_l2(got, ref) < 1e-5
+    pr.close()

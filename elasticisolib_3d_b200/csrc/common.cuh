@@ -42,15 +42,15 @@ __host__ __device__ inline int gridOfComp(int comp) {
 struct GridConst {
   int nz, nx, ny;
   int minPad;
-  long long yStride;  // nz*nx
-  long long n;        // nz*nx*ny
+  long long yStride;  // pz*nx
+  long long n;        // pz*nx*ny
   float cz[4], cx[4], cy[4];
   const float* taper;  // device, minPad entries
   int freeSurface;     // 1: free surface at z = FAT, whose face is not tapered (0: the reference's sponge)
   // y-slab of a decomposed grid: local plane y is global plane y + yOff of a grid of nyTaper
   // planes, whose y faces carry the sponge (a whole grid: yOff = 0, nyTaper = ny)
   int yOff, nyTaper;
-  int pz;  // row pitch of the fields in floats: nz, or nz rounded up (the paired stepper's padded rows)
+  int pz;  // row pitch of the fields in floats (rowLayout)
 };
 
 #ifdef __CUDACC__

@@ -68,6 +68,8 @@ struct AcqTable {
 
 struct Context {
   ContextDesc d;
+  long long cells = 0;           // nz*nx*ny, the callers' planes
+  int fieldOff = 0;              // floats between a field's allocation and its first cell
   cudaStream_t st = nullptr;     // stream all work is queued on
   cudaStream_t own = nullptr;    // the context's own stream
   GridConst g{};
@@ -101,10 +103,6 @@ struct Context {
     float* outR = nullptr;
     int its = 0, k = 0;
   } pending;
-  // nonlinear propagation of a grid whose rows are no multiple of four cells: the same grid in rows
-  // rounded up, which the TMA stepper takes (its medium a copy of this context's)
-  Context* padded = nullptr;
-  bool paddedMedium = false;
   std::unordered_map<unsigned long long, CUtensorMap> tmaps;  // (pointer, box) -> tensor map
   std::vector<void*> owned;  // every device allocation of this context
   // working wavefields (primary propagation)
@@ -174,10 +172,44 @@ static void devFree(Context* c, void* p) {
   cudaFreeAsync(p, c->st);
 }
 
+// Rows of the context's own fields and medium (the callers' planes and positions are in unpadded
+// rows).  A row is a multiple of 32 floats and starts 28 floats into its allocation, so that the first
+// updated cell (z = FAT) and every 32-cell tile row after it are whole 128-byte lines; in unpadded rows
+// a tile row starts 16 bytes into a sector and each store and box touches one more.  Measured on B200,
+// a forward step: 392x392x388 cells 1478 -> 1354 us, 168x200x188 149.7 -> 135.2; the offset of a
+// sector alone (4 floats, unpadded rows) gives 1410 and 140.9.  It costs 8 to 31 floats a row, which
+// grids holding more than 8 % of the device's memory in levels and medium do without, so that what fits
+// the device fits it still.
+static void rowLayout(const ContextDesc& d, size_t deviceBytes, int& pitch, int& offset) {
+  const double held = 26.0 * sizeof(float) * d.nz * d.nx * d.ny;
+  if (held > 0.08 * (double)deviceBytes) {
+    pitch = (d.nz + 3) / 4 * 4;
+    offset = 4;
+    return;
+  }
+  pitch = (d.nz + 31) / 32 * 32;
+  offset = 32 - FAT;
+}
+
+// A field (or `count` consecutive ones) in the context's rows.
+static int fieldAlloc(Context* c, float** p, size_t count = 1) {
+  float* raw = nullptr;
+  E3D_RET(devAlloc(c, (void**)&raw, (count * (size_t)c->g.n + c->fieldOff) * sizeof(float)));
+  *p = raw + c->fieldOff;
+  return E3D_OK;
+}
+static void fieldFree(Context* c, float* p) {
+  if (p) devFree(c, p - c->fieldOff);
+}
+
 static int allocFields(Context* c, Fields9& f, bool zero) {
   const size_t bytes = (size_t)c->g.n * sizeof(float);
   for (int k = 0; k < NCOMP; k++) {
-    if (!f.p[k]) E3D_RET(devAlloc(c, (void**)&f.p[k], bytes));
+    if (!f.p[k]) {
+      E3D_RET(fieldAlloc(c, &f.p[k]));
+      // cells no kernel writes (the ring around the grid, the rows' ends) read as zero
+      if (!zero) E3D_CUDA_TRY(cudaMemsetAsync(f.p[k], 0, bytes, c->st));
+    }
     if (zero) E3D_CUDA_TRY(cudaMemsetAsync(f.p[k], 0, bytes, c->st));
   }
   return E3D_OK;
@@ -226,10 +258,15 @@ int createContext(const ContextDesc& d, Context** out) {
   GridConst& g = c->g;
   g.nz = d.nz; g.nx = d.nx; g.ny = d.ny; g.minPad = d.minPad;
   g.yOff = 0; g.nyTaper = d.ny;
-  g.pz = d.nz;
+  {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) total = 0;
+    rowLayout(d, total, g.pz, c->fieldOff);
+  }
   g.freeSurface = d.freeSurface ? 1 : 0;
-  g.yStride = (long long)d.nz * d.nx;
+  g.yStride = (long long)g.pz * d.nx;
   g.n = g.yStride * d.ny;
+  c->cells = (long long)d.nz * d.nx * d.ny;
   // FD coefficients (nonlinearPropElasticGpuFunctions_3D.cu:207-220): double
   // quotients stored as float; y uses dx unless fixQ1 (quirk Q1).
   const double k[4] = {1.196289062541883, -0.079752604188901, 0.009570312506634, -6.975446437140719e-04};
@@ -282,10 +319,6 @@ void destroyContext(Context* c) {
     c->evPool.push_back(t.b);
   }
   for (cudaEvent_t e : c->evPool) cudaEventDestroy(e);
-  if (c->padded) {
-    c->padded->st = c->st;
-    destroyContext(c->padded);
-  }
   for (void* p : c->owned) cudaFreeAsync(p, c->st);
   c->owned.clear();
   if (c->st) cudaStreamSynchronize(c->st);
@@ -313,19 +346,29 @@ double deviceBytesInUse(const Context* c) {
 int setMedium(Context* c, const float* const* planes, bool onDevice) {
   E3D_ARG(c && planes, "null argument");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
-  const size_t bytes = (size_t)c->g.n * sizeof(float);
+  const size_t bytes = (size_t)c->cells * sizeof(float), row = (size_t)c->d.nz * sizeof(float);
   for (int k = 0; k < NMED; k++) {
     E3D_ARG(planes[k] != nullptr, "null medium plane");
-    if (!c->med[k]) E3D_RET(devAlloc(c, (void**)&c->med[k], bytes));
-    E3D_CUDA_TRY(cudaMemcpyAsync(c->med[k], planes[k], bytes, onDevice ? cudaMemcpyDeviceToDevice
-                                                                        : cudaMemcpyHostToDevice, c->st));
+    if (!c->med[k]) E3D_RET(fieldAlloc(c, &c->med[k]));
+    const float* src = planes[k];
+    if (!onDevice && c->g.pz != c->d.nz) {
+      // one copy over the bus, then the rows apart on the device
+      E3D_RET(scratchAtLeast(c, bytes));
+      E3D_CUDA_TRY(cudaMemcpyAsync(c->scratch, src, bytes, cudaMemcpyHostToDevice, c->st));
+      src = (const float*)c->scratch;
+    }
+    if (c->g.pz != c->d.nz)
+      E3D_CUDA_TRY(cudaMemcpy2DAsync(c->med[k], (size_t)c->g.pz * sizeof(float), src, row, row,
+                                     (size_t)c->d.nx * c->d.ny, cudaMemcpyDeviceToDevice, c->st));
+    else
+      E3D_CUDA_TRY(cudaMemcpyAsync(c->med[k], src, bytes, onDevice ? cudaMemcpyDeviceToDevice
+                                                                   : cudaMemcpyHostToDevice, c->st));
   }
   E3D_CUDA_TRY(cudaStreamSynchronize(c->st));
   c->haveMedium = true;
   c->ckptValid = false;
   c->tailValid = false;
   c->premCond = -1.0;
-  c->paddedMedium = false;
   return E3D_OK;
 }
 
@@ -595,7 +638,7 @@ static PairShape pairShape(const Context* c, int shots) {
 
 // The paired stepper takes every forward and time-reversed step that fuses no decimation.
 static bool pairPath(const Context* c, int mode, const StepPtrs& p) {
-  return c->loader == 8 && mode != STEP_ADJ_EXACT && c->g.pz % 4 == 0 && p.accL[0] == nullptr;
+  return c->loader == 8 && mode != STEP_ADJ_EXACT && p.accL[0] == nullptr;
 }
 
 // Paired split stepper (two z cells per thread, blockDim TZ/2 x 8), with the injection and recording
@@ -908,12 +951,15 @@ static int launchStepRaw(Context* c, int mode, const StepPtrs& p, const StepTail
     const StepTail none{};
     const StepTail& t = tail ? *tail : none;
     if (p.ssL[0]) {
-      if (mode == STEP_FWD) return launchPair<STEP_FWD, 3, 3, false, true, false>(c, p, t, 1);
+      // an odd row's last pair holds one cell (EDGE)
+      if (mode == STEP_FWD)
+        return g.nz % 2 ? launchPair<STEP_FWD, 3, 3, false, true, true>(c, p, t, 1)
+                        : launchPair<STEP_FWD, 3, 3, false, true, false>(c, p, t, 1);
     } else {
       return mode == STEP_FWD ? launchPairVariant<STEP_FWD>(c, p, t) : launchPairVariant<STEP_ADJ_REVERSED>(c, p, t);
     }
   }
-  if ((c->loader == 6 || (c->loader == 7 && mode != STEP_ADJ_EXACT)) && g.nz % 4 == 0 && p.accL[0] == nullptr &&
+  if ((c->loader == 6 || (c->loader == 7 && mode != STEP_ADJ_EXACT)) && p.accL[0] == nullptr &&
       p.ssL[0] == nullptr) {
     const int tixS = (g.nx - 2 * FAT + 7) / 8;
     if (mode == STEP_FWD) E3D_RET(launchSplitVariant<STEP_FWD>(c, p, tiz, tixS, nyi));
@@ -932,9 +978,8 @@ static int launchStepRaw(Context* c, int mode, const StepPtrs& p, const StepTail
   const int yChunk = (nyi + chunks - 1) / chunks;
   chunks = (nyi + yChunk - 1) / yChunk;
   dim3 grid(tiz, tix, chunks);
-  const bool pipe = (g.nz % 4 == 0) && mode != STEP_ADJ_EXACT && c->loader > 0;
+  const bool pipe = mode != STEP_ADJ_EXACT && c->loader > 0;
   if (dual) {
-    E3D_ARG(g.nz % 4 == 0, "dual-state adjoint needs nz % 4 == 0");
     if (c->tx == 16) E3D_RET((launchTma<STEP_ADJ_EXACT, 16, 2>(c, p, grid, yChunk)));
     else if (c->stages == 3 && c->loader < 6) E3D_RET((launchTma<STEP_ADJ_EXACT, 8, 3>(c, p, grid, yChunk)));
     else E3D_RET((launchTma<STEP_ADJ_EXACT, 8, 2>(c, p, grid, yChunk)));
@@ -1063,7 +1108,7 @@ static int launchRefresh(Context* c, const StepPtrs& p, const DevSignals& s) {
   const int n = s.off[NCOMP];
   if (n == 0) return E3D_OK;
   c->launches++;
-  kRefreshPremultiplied<<<(n + 127) / 128, 128, 0, c->st>>>(p, ss);
+  kRefreshPremultiplied<<<(n + 127) / 128, 128, 0, c->st>>>(p, c->g, ss);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
@@ -1154,8 +1199,8 @@ static int stageGeom(Context* c, const HostGeom& g, bool receivers, Staged& s) {
     E3D_ARG(n == 0 || src != nullptr, "null position table");
     for (long long i = 0; i < n; i++) {
       const long long p = src[i];
-      E3D_ARG(p >= 0 && p < c->g.n, "acquisition point outside the grid");
-      const long long iz = p % c->d.nz, ix = (p / c->d.nz) % c->d.nx, iy = p / c->g.yStride;
+      E3D_ARG(p >= 0 && p < c->cells, "acquisition point outside the grid");
+      const long long iz = p % c->d.nz, ix = (p / c->d.nz) % c->d.nx, iy = p / ((long long)c->d.nz * c->d.nx);
       if (iz < FAT || iz >= c->d.nz - FAT || ix < FAT || ix >= c->d.nx - FAT || iy < FAT || iy >= c->d.ny - FAT) {
         setLastError("acquisition point inside the FAT ring", __FILE__, __LINE__);
         return E3D_ERR_BOUNDS;
@@ -1254,7 +1299,7 @@ static int launchRecordIdx(Context* c, const StepPtrs& p, const DevSignals& s, f
 }
 
 // Whether the passes of this context can leave injection and recording to the stepper launch.
-static bool takesTail(const Context* c) { return c->loader == 8 && c->g.pz % 4 == 0; }
+static bool takesTail(const Context* c) { return c->loader == 8; }
 
 // One coarse block of the nonlinear loops.  Forward (propElasticFwdGpu_3D):
 // per fine step it2 = 1..sub  step -> inject (k=it2-1) -> [free surface] ->
@@ -1461,14 +1506,14 @@ int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const 
   const size_t bytes = (size_t)shots * c->g.n * sizeof(float);
   if (c->batchShots != shots) {
     for (int k = 0; k < NCOMP; k++) {
-      devFree(c, c->bw0.p[k]);
-      devFree(c, c->bw1.p[k]);
+      fieldFree(c, c->bw0.p[k]);
+      fieldFree(c, c->bw1.p[k]);
       c->bw0.p[k] = c->bw1.p[k] = nullptr;
     }
     c->batchShots = 0;
     for (int k = 0; k < NCOMP; k++) {
-      E3D_RET(devAlloc(c, (void**)&c->bw0.p[k], bytes));
-      E3D_RET(devAlloc(c, (void**)&c->bw1.p[k], bytes));
+      E3D_RET(fieldAlloc(c, &c->bw0.p[k], shots));
+      E3D_RET(fieldAlloc(c, &c->bw1.p[k], shots));
     }
     c->batchShots = shots;
   }
@@ -1520,72 +1565,10 @@ int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const 
   return flushRecord(c, c->bw1, recSet, true);
 }
 
-// The context of the same grid in rows of a multiple of four cells, with this context's medium; *out
-// null where the device has no memory for it (the grid then runs on the plain stepper).
-static int paddedContext(Context* c, Context** out) {
-  *out = nullptr;
-  Context* t = c->padded;
-  if (!t) {
-    t = new Context();
-    t->d = c->d;
-    t->g = c->g;
-    t->g.pz = (c->d.nz + 3) / 4 * 4;
-    t->g.yStride = (long long)t->g.pz * c->d.nx;
-    t->g.n = t->g.yStride * c->d.ny;
-    t->hfilt = c->hfilt;
-    t->filt = c->filt;
-    t->dtsInv = c->dtsInv;
-    t->numSMs = c->numSMs;
-    t->haveMedium = true;
-    c->padded = t;
-    c->paddedMedium = false;
-  }
-  t->st = c->st;
-  t->stages = c->stages;
-  t->yChunks = c->yChunks;
-  t->graphLoop = c->graphLoop;
-  t->timingEvery = c->timingEvery;
-  int st = E3D_OK;
-  for (int k = 0; k < NMED && st == E3D_OK; k++)
-    if (!t->med[k]) st = devAlloc(t, (void**)&t->med[k], (size_t)t->g.n * sizeof(float));
-  if (st == E3D_OK) st = allocFields(t, t->w0, false);
-  if (st == E3D_OK) st = allocFields(t, t->w1, false);
-  if (st == E3D_ERR_OOM) {
-    cudaGetLastError();
-    destroyContext(t);
-    c->padded = nullptr;
-    return E3D_OK;
-  }
-  E3D_RET(st);
-  if (!c->paddedMedium) {
-    for (int k = 0; k < NMED; k++)
-      E3D_CUDA_TRY(cudaMemcpy2DAsync(t->med[k], (size_t)t->g.pz * sizeof(float), c->med[k],
-                                     (size_t)c->d.nz * sizeof(float), (size_t)c->d.nz * sizeof(float),
-                                     (size_t)c->d.nx * c->d.ny, cudaMemcpyDeviceToDevice, c->st));
-    c->paddedMedium = true;
-  }
-  *out = t;
-  return E3D_OK;
-}
-
 int nlPropagateDevice(Context* c, bool adjoint, const DevSignals& srcSet, const DevSignals& recSet, float* srcSig,
                       float* recSig) {
   E3D_ARG(c && c->haveMedium, "medium not set");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
-  if (c->loader == 8 && c->g.pz % 4 != 0) {
-    // rows that no bulk copy can start on: the same grid in rounded-up rows.  Measured on B200 at
-    // 101 x 91 x 117 cells against the plain stepper: see kStepSplitPair
-    Context* t = nullptr;
-    E3D_RET(paddedContext(c, &t));
-    if (t) {
-      const long long before = t->launches;
-      const int st = nlPropagateDevice(t, adjoint, srcSet, recSet, srcSig, recSig);
-      c->launches += t->launches - before;
-      c->timed.insert(c->timed.end(), t->timed.begin(), t->timed.end());
-      t->timed.clear();
-      return st;
-    }
-  }
   E3D_RET(allocFields(c, c->w0, true));
   E3D_RET(allocFields(c, c->w1, true));
   c->tailReady = takesTail(c);
@@ -1695,11 +1678,17 @@ int stageSlabTables(Context* c, const std::vector<long long>* pos, Staged& s) {
 // Copy planes [from, from + FAT) of the nine fields of `src` into planes [to, to + FAT) of `dst`
 // on dst's stream (peer copies between devices through unified addressing).
 int copyGhostPlanes(const SlabRun& dst, long long to, const SlabRun& src, long long from) {
-  const long long ys = dst.c->g.yStride;
-  const size_t bytes = (size_t)FAT * ys * sizeof(float);
-  for (int k = 0; k < NCOMP; k++)
-    E3D_CUDA_TRY(cudaMemcpyAsync(dst.c->w1.p[k] + to * ys, src.c->w1.p[k] + from * ys, bytes, cudaMemcpyDefault,
-                                 dst.c->st));
+  const GridConst &a = dst.c->g, &b = src.c->g;
+  const size_t row = (size_t)a.nz * sizeof(float);
+  for (int k = 0; k < NCOMP; k++) {
+    float* to_ = dst.c->w1.p[k] + to * a.yStride;
+    const float* from_ = src.c->w1.p[k] + from * b.yStride;
+    if (a.pz == b.pz)  // whole planes
+      E3D_CUDA_TRY(cudaMemcpyAsync(to_, from_, (size_t)FAT * a.yStride * sizeof(float), cudaMemcpyDefault, dst.c->st));
+    else
+      E3D_CUDA_TRY(cudaMemcpy2DAsync(to_, (size_t)a.pz * sizeof(float), from_, (size_t)b.pz * sizeof(float), row,
+                                     (size_t)FAT * a.nx, cudaMemcpyDefault, dst.c->st));
+  }
   return E3D_OK;
 }
 }  // namespace
@@ -1727,7 +1716,7 @@ int nlPropagateSlabsHost(Context* const* slabs, int nSlabs, int nyGlobal, bool a
     y += d.ny - 2 * FAT;
   }
   E3D_ARG(y + 2 * FAT == nyGlobal, "slab sizes do not add up to ny (sum of ny_domDec - 2*FAT*(n-1) != ny)");
-  const long long ys = c0->g.yStride;
+  const long long ys = (long long)c0->d.nz * c0->d.nx;  // a plane of the callers' positions
   const long long nG = ys * nyGlobal;
 
   // deal the acquisition points to the slabs that update them
@@ -1895,7 +1884,7 @@ int stepOnly(Context* c, int mode, int nSteps) {
     E3D_RET(allocFields(c, c->ss[1], true));
   }
   // the exact adjoint runs on the dual state, as in the adjoint pass, with the TMA loader
-  const bool dual = m == STEP_ADJ_EXACT && c->loader >= 2 && c->d.nz % 4 == 0;
+  const bool dual = m == STEP_ADJ_EXACT && c->loader >= 2;
   if (dual) {
     E3D_RET(allocFields(c, c->q0, false));
     E3D_RET(allocFields(c, c->q1, false));
@@ -1931,7 +1920,7 @@ int checkpointSegment(const Context* c) { return c->ckptSegLen; }
 static int ensureVSlots(Context* c, int nslots) {
   while ((int)c->vSlots.size() < nslots) {
     float* v = nullptr;
-    E3D_RET(devAlloc(c, (void**)&v, (size_t)3 * c->g.n * sizeof(float)));
+    E3D_RET(fieldAlloc(c, &v, 3));
     c->vSlots.push_back(v);
   }
   return E3D_OK;
@@ -2017,7 +2006,7 @@ constexpr double kPremCondMax = 100.0;
 
 static int premultipliedAdjoint(Context* c, bool& use) {
   use = false;
-  if (!c->premMode || c->loader < 2 || c->d.nz % 4 != 0 || !c->haveMedium) return E3D_OK;
+  if (!c->premMode || c->loader < 2 || !c->haveMedium) return E3D_OK;
   if (c->premCond < 0) {
     if (!c->posFlag) E3D_RET(devAlloc(c, (void**)&c->posFlag, sizeof(unsigned)));
     E3D_CUDA_TRY(cudaMemsetAsync(c->posFlag, 0, sizeof(unsigned), c->st));
@@ -2048,7 +2037,7 @@ static Fields9& ringAt(std::vector<Fields9>& r, long long m) {
   return r[(size_t)(((m % R) + R) % R)];
 }
 
-// Allocate a ring of `levels` levels whose first two are a and b; every level zeroed.
+// Allocate a ring of `levels` levels whose first two are a and b; levels -1 and 0 zeroed.
 static int ensureRing(Context* c, std::vector<Fields9>& ring, Fields9& a, Fields9& b, int levels) {
   if (ring.empty()) {
     E3D_RET(allocFields(c, a, false));
@@ -2062,8 +2051,9 @@ static int ensureRing(Context* c, std::vector<Fields9>& ring, Fields9& a, Fields
     }
   }
   E3D_ARG((int)ring.size() == levels, "ring size changed");
-  for (auto& f : ring) E3D_RET(zeroFields(c, f));
-  return E3D_OK;
+  // levels -1 and 0; a step writes every updated cell of the others before it is read
+  E3D_RET(zeroFields(c, ring.back()));
+  return zeroFields(c, ring.front());
 }
 
 // Source velocity of the block whose last fine level is mEnd (fine steps 1..sub
@@ -2187,12 +2177,11 @@ static int launchImagingBlock(Context* c, long long mEnd, float* const v[4], boo
   q.q3compat = c->d.q3compat;
   c->launches++;
   TimedLaunch tl(c, 6);
-  const bool tma = c->d.nz % 4 == 0 && c->loader >= 2;
+  const bool tma = c->loader >= 2;
   int variant = c->imgVariant;
   // automatic: the y-march with velocity tiles staged by TMA.  Measured on B200 in the 288^3
   // gradient: 1.46 ms per block against 1.88 ms with the levels staged too (one CTA per SM)
   if (variant == 0) variant = tma ? 2 : 1;
-  if (variant >= 2 && c->d.nz % 4 != 0) variant = 1;  // the TMA forms need 16-byte rows
   const int tiz = (c->g.nz - 2 * FAT + TZ - 1) / TZ;
   const int tix = (c->g.nx - 2 * FAT + IMG_TX - 1) / IMG_TX;
   const int nyi = c->g.ny - 2 * FAT;
@@ -2222,7 +2211,7 @@ static int launchImagingBlock(Context* c, long long mEnd, float* const v[4], boo
 
 static int ensurePert(Context* c) {
   for (int k = 0; k < NMED; k++)
-    if (!c->pertDev[k]) E3D_RET(devAlloc(c, (void**)&c->pertDev[k], (size_t)c->g.n * sizeof(float)));
+    if (!c->pertDev[k]) E3D_RET(devAlloc(c, (void**)&c->pertDev[k], (size_t)c->cells * sizeof(float)));
   return E3D_OK;
 }
 
@@ -2387,7 +2376,7 @@ static int choosePlan(Context* c, int& L) {
 
 static int resizeVStorage(Context* c, int nF32, int nF16) {
   while ((int)c->vSlots.size() > nF32) {
-    devFree(c, c->vSlots.back());
+    fieldFree(c, c->vSlots.back());
     c->vSlots.pop_back();
   }
   while ((int)c->vStore.size() > nF16) {
@@ -2657,7 +2646,7 @@ static int adjointPassFromCheckpoints(Context* c, const DevSignals& srcSet, cons
   E3D_RET(allocFields(c, c->ss[0], true));
   E3D_RET(allocFields(c, c->ss[1], true));
   // the TMA stepper runs the exact adjoint on a dual state (raw + premultiplied)
-  const bool dual = c->loader >= 2 && c->d.nz % 4 == 0;
+  const bool dual = c->loader >= 2;
   if (dual) {
     E3D_RET(allocFields(c, c->q0, true));
     E3D_RET(allocFields(c, c->q1, true));
@@ -2911,7 +2900,7 @@ static int adjointPassRing(Context* c, const DevSignals& srcSet, const DevSignal
   E3D_RET(ensureRing(c, c->adjRing, c->w0, c->w1, ringLevels(c)));
   Fields9& carry = c->ss[0];
   E3D_RET(allocFields(c, carry, true));  // L of the block after the last one: zero
-  const bool dual = c->loader >= 2 && c->d.nz % 4 == 0;
+  const bool dual = c->loader >= 2;
   // the premultiplied-only state: the ring holds premultiplied levels and no raw level is kept
   bool prem = false;
   const int ncn = recSet.off[SXX + 1] - recSet.off[SXX];
@@ -3054,7 +3043,7 @@ int bornForwardHost(Context* c, const float* const* srcSig, float* const* data, 
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
   E3D_RET(ensurePert(c));
   for (int k = 0; k < NMED; k++)
-    E3D_CUDA_TRY(cudaMemcpyAsync(c->pertDev[k], pert[k], (size_t)c->g.n * sizeof(float), cudaMemcpyHostToDevice,
+    E3D_CUDA_TRY(cudaMemcpyAsync(c->pertDev[k], pert[k], (size_t)c->cells * sizeof(float), cudaMemcpyHostToDevice,
                                  c->st));
   Staged S, R;
   int st = stageGeom(c, src, false, S);
@@ -3083,7 +3072,7 @@ int bornAdjointHost(Context* c, const float* const* srcSig, const float* const* 
   // the reference copies the caller's planes to the device and accumulates
   // the image onto them (BornElasticGpuFunctions_3D.cu:2110-2114)
   for (int k = 0; k < NMED; k++)
-    E3D_CUDA_TRY(cudaMemcpyAsync(c->pertDev[k], pert[k], (size_t)c->g.n * sizeof(float), cudaMemcpyHostToDevice,
+    E3D_CUDA_TRY(cudaMemcpyAsync(c->pertDev[k], pert[k], (size_t)c->cells * sizeof(float), cudaMemcpyHostToDevice,
                                  c->st));
   Staged S, R;
   int st = stageGeom(c, src, false, S);
@@ -3094,7 +3083,7 @@ int bornAdjointHost(Context* c, const float* const* srcSig, const float* const* 
   if (st == E3D_OK) st = checkPipeError(c);
   if (st == E3D_OK) {
     for (int k = 0; k < NMED && st == E3D_OK; k++) {
-      cudaError_t e = cudaMemcpyAsync(pert[k], c->pertDev[k], (size_t)c->g.n * sizeof(float),
+      cudaError_t e = cudaMemcpyAsync(pert[k], c->pertDev[k], (size_t)c->cells * sizeof(float),
                                       cudaMemcpyDeviceToHost, c->st);
       if (e != cudaSuccess) st = E3D_ERR_CUDA;
     }

@@ -47,6 +47,11 @@ struct SparseSet {
   int off[NCOMP + 1];
 };
 
+// Cell (z, x, y) of an image or perturbation plane, which is the caller's: unpadded rows.
+__device__ __forceinline__ long long planeCell(const GridConst& g, int iz, int ix, int iy) {
+  return ((long long)iy * g.nx + ix) * g.nz + iz;
+}
+
 // Cell of a position given in unpadded rows (stacked shots carry shot * nz*nx*ny).
 __device__ __forceinline__ long long cellIndex(const GridConst& g, long long pos) {
   return g.pz == g.nz ? pos : pos / g.nz * g.pz + pos % g.nz;
@@ -149,7 +154,7 @@ __global__ void __launch_bounds__(TZ * TX) kStep(StepPtrs p, GridConst g, int yC
   const int yBeg = FAT + blockIdx.z * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz;
 
   float w[NQUEUE][8];
   if (active) {
@@ -181,7 +186,7 @@ __global__ void __launch_bounds__(TZ * TX) kStep(StepPtrs p, GridConst g, int yC
         const int lz = s % SZ, lx = s / SZ;
         const int gz = z0 - HALO + lz, gx = x0 - HALO + lx;
         const bool in = (gz < g.nz) && (gx < g.nx);
-        const long long gi = plane + (long long)gx * g.nz + gz;
+        const long long gi = plane + (long long)gx * g.pz + gz;
 #pragma unroll
         for (int t = 0; t < NTILE; t++) tile[t][s] = in ? tileValue<MODE>(p, t, gi) : 0.0f;
       }
@@ -246,8 +251,7 @@ __global__ void __launch_bounds__(TZ * TX) kStep(StepPtrs p, GridConst g, int yC
 // global read (the eight halo tiles, the six y-window leads, the old level and
 // the medium) is issued as 16-byte cp.async copies into a STAGES-deep ring of
 // shared-memory stages, so plane y+1.. are in flight while plane y computes,
-// with one barrier per plane.  Requires nz % 4 == 0 (16-byte rows), which the
-// reference's block-size rule guarantees.
+// with one barrier per plane.  Requires 16-byte rows (rowLayout's).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cpAsync16(float* smem, const float* gmem, bool valid) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -289,7 +293,7 @@ __device__ __forceinline__ void issuePlane(const StepPtrs& p, const GridConst& g
   constexpr int NT = TZ * TX;
   const long long ys = g.yStride;
   const long long plane = (long long)y * ys;
-  // halo tiles: rows of 40 floats starting at z0-4 (16-byte aligned when nz % 4 == 0)
+  // halo tiles: rows of 40 floats starting at z0-4 (16-byte aligned: rowLayout)
   for (int c = tid; c < NTILE * L::HALO_CH; c += NT) {
     const int t = c / L::HALO_CH;
     const int r = c - t * L::HALO_CH;
@@ -297,7 +301,7 @@ __device__ __forceinline__ void issuePlane(const StepPtrs& p, const GridConst& g
     const int gz = z0 - HALO + 4 * q, gx = x0 - HALO + lx;
     const bool ok = (gz < g.nz) && (gx < g.nx);
     const float* src = p.c[tileComp(t)];
-    cpAsync16(st + t * L::HALO_F + lx * SZ + 4 * q, ok ? src + plane + (long long)gx * g.nz + gz : src, ok);
+    cpAsync16(st + t * L::HALO_F + lx * SZ + 4 * q, ok ? src + plane + (long long)gx * g.pz + gz : src, ok);
   }
   // interior tiles: y-window leads, old level, medium
   for (int c = tid; c < L::N_INT * L::INT_CH; c += NT) {
@@ -307,7 +311,7 @@ __device__ __forceinline__ void issuePlane(const StepPtrs& p, const GridConst& g
     const int gz = z0 + 4 * q, gx = x0 + lx;
     const bool ok = (gz < g.nz) && (gx < g.nx);
     const float* src;
-    long long off = (long long)gx * g.nz + gz;
+    long long off = (long long)gx * g.pz + gz;
     if (f < NQUEUE) {
       src = p.c[queueComp(f)];
       off += (long long)(y + qBase(f) + 7) * ys;
@@ -334,7 +338,7 @@ __global__ void __launch_bounds__(TZ * TX) kStepPipe(StepPtrs p, GridConst g, in
   const int yBeg = FAT + blockIdx.z * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz;
 
   // prologue: planes yBeg .. yBeg+STAGES-2 in flight
 #pragma unroll
@@ -516,7 +520,7 @@ __global__ void __launch_bounds__(TZ * TX) kStepTma(const __grid_constant__ TmaM
   const int yBeg = FAT + blockIdx.z * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz;
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) mbarInit(&bars[s], 1);
@@ -741,7 +745,7 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
   const int yBeg = FAT + chunk * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz;
   if (tid == 0) {
     for (int s = 0; s < STAGES; s++) mbarInit(&bars[s], 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -1390,7 +1394,7 @@ __global__ void __launch_bounds__(TZ * 8, MINB) kStepSplit(const __grid_constant
 // Recompute the premultiplied level at injected points (dual-state mode 2):
 // after kInject changed raw values there.  The three normal stresses share
 // the center-grid positions and are refreshed together by the sxx entries.
-__global__ void kRefreshPremultiplied(StepPtrs p, SparseSet s) {
+__global__ void kRefreshPremultiplied(StepPtrs p, GridConst g, SparseSet s) {
   const int ntot = s.off[NCOMP];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ntot) return;
@@ -1398,7 +1402,7 @@ __global__ void kRefreshPremultiplied(StepPtrs p, SparseSet s) {
 #pragma unroll
   for (int c = 1; c < NCOMP; c++) k += (j >= s.off[c]);
   if (k == SYY || k == SZZ) return;
-  const long long i = s.pos[j];
+  const long long i = cellIndex(g, s.pos[j]);
   switch (k) {
     case VX: p.oP[VX][i] = p.o[VX][i] * __ldg(p.m[RHOX] + i); break;
     case VY: p.oP[VY][i] = p.o[VY][i] * __ldg(p.m[RHOY] + i); break;
@@ -1431,10 +1435,10 @@ __global__ void kInjectRefresh(StepPtrs p, GridConst g, SparseSet s, const float
 #pragma unroll
   for (int c = 1; c < NCOMP; c++) k += (j >= s.off[c]);
   if (k == SYY || k == SZZ) return;
-  const long long i = s.pos[j];
-  const int iz = (int)(i % g.nz);
-  const int ix = (int)((i / g.nz) % g.nx);
-  const int iy = (int)(i / g.yStride);
+  const long long pos = s.pos[j], i = cellIndex(g, pos);
+  const int iz = (int)(pos % g.nz);
+  const int ix = (int)((pos / g.nz) % g.nx);
+  const int iy = (int)(pos / ((long long)g.nz * g.nx));
   const float G = taperAt(g, iz, ix, iy);
   if (k == SXX) {
     const int r = j - s.off[SXX];
@@ -1471,10 +1475,10 @@ __global__ void kInjectPremultiplied(StepPtrs p, GridConst g, SparseSet s, const
 #pragma unroll
   for (int c = 1; c < NCOMP; c++) k += (j >= s.off[c]);
   if (k == SYY || k == SZZ) return;
-  const long long i = s.pos[j];
-  const int iz = (int)(i % g.nz);
-  const int ix = (int)((i / g.nz) % g.nx);
-  const int iy = (int)(i / g.yStride);
+  const long long pos = s.pos[j], i = cellIndex(g, pos);
+  const int iz = (int)(pos % g.nz);
+  const int ix = (int)((pos / g.nz) % g.nx);
+  const int iy = (int)(pos / ((long long)g.nz * g.nx));
   const float G = taperAt(g, iz, ix, iy);
   if (k == SXX) {
     const int r = j - s.off[SXX];
@@ -1504,8 +1508,8 @@ __global__ void kPremultiplyCondition(StepPtrs p, GridConst g, unsigned* out) {
   float worst = 0.0f;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ncell;
        i += (long long)gridDim.x * blockDim.x) {
-    const int iz = (int)(i % g.nz);
-    const int ix = (int)((i / g.nz) % g.nx);
+    const int iz = (int)(i % g.pz);
+    const int ix = (int)((i / g.pz) % g.nx);
     const int iy = (int)(i / g.yStride);
     if (iz < FAT || iz >= g.nz - FAT || ix < FAT || ix >= g.nx - FAT || iy < FAT || iy >= g.ny - FAT) continue;
     const float a = __ldg(m[L2M] + i), b = __ldg(m[LAM] + i);
@@ -1686,7 +1690,7 @@ __global__ void __launch_bounds__(TZ * TX, MINB) kStepTma2(const __grid_constant
   S.active = (S.iz < g.nz - FAT) && (S.ix < g.nx - FAT);
   const int yBeg = FAT + blockIdx.z * yChunk;
   S.yEnd = min(yBeg + yChunk, g.ny - FAT);
-  S.col = (long long)S.ix * g.nz + S.iz;
+  S.col = (long long)S.ix * g.pz + S.iz;
   S.dzx = min(min(topDistance(g, S.iz), S.ix - FAT), min(g.nz - S.iz - 1 - FAT, g.nx - S.ix - 1 - FAT));
   S.lc = (tx + HALO) * SZ + (tz + HALO);
   S.li = tx * TZ + tz;
@@ -1840,9 +1844,9 @@ __global__ void kFreeSurface(StepPtrs p, GridConst g, float sgn) {
   const int iy = FAT + blockIdx.y;
   if (ix >= g.nx - FAT || iy >= g.ny - FAT) return;
   const long long ys = g.yStride;
-  const long long col = (long long)iy * ys + (long long)ix * g.nz;
+  const long long col = (long long)iy * ys + (long long)ix * g.pz;
   const long long i = col + FAT;
-  const float dvx = dPlusG(p.c[VX], i, g.nz, g.cx);
+  const float dvx = dPlusG(p.c[VX], i, g.pz, g.cx);
   const float dvy = dPlusG(p.c[VY], i, ys, g.cy);
   const float dvz = dPlusG(p.c[VZ], i, 1, g.cz);
   const float l2m = __ldg(p.m[L2M] + i), lam = __ldg(p.m[LAM] + i);
@@ -1892,8 +1896,8 @@ __global__ void kExtractSource(StepPtrs p, GridConst g, SparseSet s, float* outL
   const long long pos = s.pos[j];
   const int iz = (int)(pos % g.nz);
   const int ix = (int)((pos / g.nz) % g.nx);
-  const int iy = (int)((pos / g.yStride) % g.ny);  // positions of stacked shots carry shot * n
-  const float v = taperAt(g, iz, ix, iy) * p.o[k][pos];
+  const int iy = (int)((pos / ((long long)g.nz * g.nx)) % g.ny);  // positions of stacked shots carry shot * n
+  const float v = taperAt(g, iz, ix, iy) * p.o[k][cellIndex(g, pos)];
   outL[j] += v * wl;
   outR[j] += v * wr;
 }
@@ -1971,8 +1975,9 @@ __global__ void kImaging(ImagingPtrs q, GridConst g) {
   const int ix = FAT + blockIdx.y * blockDim.y + threadIdx.y;
   const int iy = FAT + blockIdx.z;
   if (iz >= g.nz - FAT || ix >= g.nx - FAT) return;
-  const long long i = (long long)iy * g.yStride + (long long)ix * g.nz + iz;
-  const long long xs = g.nz, ys = g.yStride;
+  const long long i = (long long)iy * g.yStride + (long long)ix * g.pz + iz;
+  const long long iu = planeCell(g, iz, ix, iy);
+  const long long xs = g.pz, ys = g.yStride;
   const float* vx = q.vCur[0];
   const float* vy = q.vCur[1];
   const float* vz = q.vCur[2];
@@ -1991,26 +1996,26 @@ __global__ void kImaging(ImagingPtrs q, GridConst g) {
   }
   const float div = dvx_dx + dvy_dy + dvz_dz;
   if (!ADJ) {
-    q.ss[VX][i] = __ldg(q.pert[0] + i) * tder[0];
-    q.ss[VY][i] = __ldg(q.pert[1] + i) * tder[1];
-    q.ss[VZ][i] = __ldg(q.pert[2] + i) * tder[2];
-    const float dl = __ldg(q.pert[3] + i), dm = __ldg(q.pert[4] + i);
+    q.ss[VX][i] = __ldg(q.pert[0] + iu) * tder[0];
+    q.ss[VY][i] = __ldg(q.pert[1] + iu) * tder[1];
+    q.ss[VZ][i] = __ldg(q.pert[2] + iu) * tder[2];
+    const float dl = __ldg(q.pert[3] + iu), dm = __ldg(q.pert[4] + iu);
     q.ss[SXX][i] = dl * div + 2.0f * dm * dvx_dx;
     q.ss[SYY][i] = dl * div + 2.0f * dm * dvy_dy;
     q.ss[SZZ][i] = dl * div + 2.0f * dm * dvz_dz;
-    q.ss[SXZ][i] = __ldg(q.pert[5] + i) * exz;
-    q.ss[SXY][i] = __ldg(q.pert[6] + i) * exy;
-    q.ss[SYZ][i] = __ldg(q.pert[7] + i) * eyz;
+    q.ss[SXZ][i] = __ldg(q.pert[5] + iu) * exz;
+    q.ss[SXY][i] = __ldg(q.pert[6] + iu) * exy;
+    q.ss[SYZ][i] = __ldg(q.pert[7] + iu) * eyz;
   } else {
     const float axx = q.ss[SXX][i], ayy = q.ss[SYY][i], azz = q.ss[SZZ][i];
-    q.pert[0][i] += q.ss[VX][i] * tder[0];
-    q.pert[1][i] += q.ss[VY][i] * tder[1];
-    q.pert[2][i] += q.ss[VZ][i] * tder[2];
-    q.pert[3][i] += (axx + ayy + azz) * div;
-    q.pert[4][i] += 2.0f * (dvx_dx * axx + dvy_dy * ayy + dvz_dz * azz);
-    q.pert[5][i] += q.ss[SXZ][i] * exz;
-    q.pert[6][i] += q.ss[SXY][i] * exy;
-    q.pert[7][i] += q.ss[SYZ][i] * eyz;
+    q.pert[0][iu] += q.ss[VX][i] * tder[0];
+    q.pert[1][iu] += q.ss[VY][i] * tder[1];
+    q.pert[2][iu] += q.ss[VZ][i] * tder[2];
+    q.pert[3][iu] += (axx + ayy + azz) * div;
+    q.pert[4][iu] += 2.0f * (dvx_dx * axx + dvy_dy * ayy + dvz_dz * azz);
+    q.pert[5][iu] += q.ss[SXZ][i] * exz;
+    q.pert[6][iu] += q.ss[SXY][i] * exy;
+    q.pert[7][iu] += q.ss[SYZ][i] * eyz;
   }
 }
 
@@ -2081,7 +2086,7 @@ struct VelTerms {
 __device__ __forceinline__ VelTerms velTerms(const float* const* vPrev, const float* const* vCur,
                                              const float* const* vNext, long long i, const GridConst& g,
                                              float dtsInv, int q3compat) {
-  const long long xs = g.nz, ys = g.yStride;
+  const long long xs = g.pz, ys = g.yStride;
   const float* vx = vCur[0];
   const float* vy = vCur[1];
   const float* vz = vCur[2];
@@ -2196,7 +2201,7 @@ __global__ void __launch_bounds__(256) kImagingBlock(ImagingBlockPtrs q, GridCon
   const int ix = FAT + blockIdx.y * blockDim.y + threadIdx.y;
   const int iy = FAT + blockIdx.z;
   if (iz >= g.nz - FAT || ix >= g.nx - FAT) return;
-  const long long i = (long long)iy * g.yStride + (long long)ix * g.nz + iz;
+  const long long i = (long long)iy * g.yStride + (long long)ix * g.pz + iz;
   float L[NCOMP], R[NCOMP];
   blockSums(q, i, L, R);
   float acc[NMED];
@@ -2215,7 +2220,7 @@ __global__ void __launch_bounds__(256) kImagingBlock(ImagingBlockPtrs q, GridCon
     for (int k = 0; k < NCOMP; k++) q.carry[k][i] = L[k];
   }
 #pragma unroll
-  for (int k = 0; k < NMED; k++) q.pert[k][i] += acc[k];
+  for (int k = 0; k < NMED; k++) q.pert[k][planeCell(g, iz, ix, iy)] += acc[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -2281,7 +2286,7 @@ __global__ void __launch_bounds__(TZ * IMG_TX) kImagingTma(const __grid_constant
   const int yBeg = FAT + blockIdx.z * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz;
   const int ntimes = q.leftImage ? 2 : 1;
   const int t0 = 2 - ntimes;  // first time index present
 
@@ -2307,7 +2312,7 @@ __global__ void __launch_bounds__(TZ * IMG_TX) kImagingTma(const __grid_constant
   int slot = 0;
   unsigned parity = 0;
   for (int y = yBeg; y < yEnd; y++) {
-    const long long ic = (long long)y * ys + col;
+    const long long ic = (long long)y * ys + col, iu = planeCell(g, iz, ix, y);
     // coalesced per-cell loads, issued ahead of the wait
     float L[NCOMP], R[NCOMP], pv[NMED], nxt[3], prv[3], cur0[3];
     if (active) {
@@ -2319,7 +2324,7 @@ __global__ void __launch_bounds__(TZ * IMG_TX) kImagingTma(const __grid_constant
         cur0[k] = q.leftImage ? 0.f : __ldg(q.v[1][k] + ic);                     // V(its) without its tile
       }
 #pragma unroll
-      for (int k = 0; k < NMED; k++) pv[k] = q.pert[k][ic];
+      for (int k = 0; k < NMED; k++) pv[k] = q.pert[k][iu];
     }
     const bool ok = mbarWaitBounded(&bars[slot], (parity >> slot) & 1u);
     if (__syncthreads_or(!ok)) {
@@ -2372,7 +2377,7 @@ __global__ void __launch_bounds__(TZ * IMG_TX) kImagingTma(const __grid_constant
         for (int k = 0; k < NCOMP; k++) q.carry[k][ic] = L[k];
       }
 #pragma unroll
-      for (int k = 0; k < NMED; k++) q.pert[k][ic] = pv[k] + acc[k];
+      for (int k = 0; k < NMED; k++) q.pert[k][iu] = pv[k] + acc[k];
 #pragma unroll
       for (int t = 0; t < 2; t++)
 #pragma unroll
@@ -2451,7 +2456,7 @@ __global__ void __launch_bounds__(TZ * ITX, ITX == 4 ? 3 : 1) kImagingLev(const 
   const int yBeg = FAT + blockIdx.z * yChunk;
   const int yEnd = min(yBeg + yChunk, g.ny - FAT);
   const long long ys = g.yStride;
-  const long long col = (long long)ix * g.nz + iz;
+  const long long col = (long long)ix * g.pz + iz;
   const int ntimes = q.leftImage ? 2 : 1;
   const int t0 = 2 - ntimes;
   const bool prem = q.prem != 0;
@@ -2479,7 +2484,7 @@ __global__ void __launch_bounds__(TZ * ITX, ITX == 4 ? 3 : 1) kImagingLev(const 
   int slot = 0;
   unsigned parity = 0;
   for (int y = yBeg; y < yEnd; y++) {
-    const long long ic = (long long)y * ys + col;
+    const long long ic = (long long)y * ys + col, iu = planeCell(g, iz, ix, y);
     float pv[NMED], nxt[3], prv[3], cur0[3], cin[NCOMP];
     if (active) {
 #pragma unroll
@@ -2491,7 +2496,7 @@ __global__ void __launch_bounds__(TZ * ITX, ITX == 4 ? 3 : 1) kImagingLev(const 
 #pragma unroll
       for (int k = 0; k < NCOMP; k++) cin[k] = q.carryIn ? q.carry[k][ic] : 0.f;
 #pragma unroll
-      for (int k = 0; k < NMED; k++) pv[k] = q.pert[k][ic];
+      for (int k = 0; k < NMED; k++) pv[k] = q.pert[k][iu];
     }
     const bool ok = mbarWaitBounded(&bars[slot], (parity >> slot) & 1u);
     if (__syncthreads_or(!ok)) {
@@ -2575,7 +2580,7 @@ __global__ void __launch_bounds__(TZ * ITX, ITX == 4 ? 3 : 1) kImagingLev(const 
         for (int k = 0; k < NCOMP; k++) q.carry[k][ic] = L[k];
       }
 #pragma unroll
-      for (int k = 0; k < NMED; k++) q.pert[k][ic] = pv[k] + acc[k];
+      for (int k = 0; k < NMED; k++) q.pert[k][iu] = pv[k] + acc[k];
 #pragma unroll
       for (int t = 0; t < 2; t++)
 #pragma unroll

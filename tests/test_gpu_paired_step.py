@@ -53,3 +53,28 @@ def test_paired_step_matches_oracle(nz, nx, ny, nts, sub, nsrc, nrec, adjoint, s
             ref = O.nl_forward_reg(p, med64, sig64, spos, rpos, np.float64)
         assert rel_l2(got, ref) < 1e-5
     pr.close()
+
+
+@pytest.mark.parametrize("nz,nx,ny,nts,sub,nsrc,nrec", GRIDS)
+def test_born_pair_matches_oracle(nz, nx, ny, nts, sub, nsrc, nrec):
+    """The linearised pair on the same grids: secondary sources in the paired step, source levels
+    decimated from a ring, the image in the caller's rows (test_gpu_parity's 1e-5)."""
+    rng = np.random.default_rng(nz)
+    el = S.elastic_from_velocity(*S.gaussian_perturbed_model((ny, nx, nz), 2500.0, 1443.0, 2000.0, 0.1, 2.0, 5))
+    dts = 0.0005 * sub
+    med = O.medium_planes(el, dts / sub, np.float32)
+    p = O.PropParams(nz, nx, ny, nts, sub, 3, 10.0, 10.0, 10.0, dts)
+    spos = [_points(rng, nz, nx, ny, nsrc) for _ in range(7)]
+    rpos = [_points(rng, nz, nx, ny, nrec) for _ in range(7)]
+    sig, dat = random_signals(spos, nts, rng), random_signals(rpos, nts, rng)
+    pert = rng.standard_normal((8, ny, nx, nz)).astype(np.float32)
+    pr = Propagator(nz, nx, ny, nts, sub, 3, 10.0, 10.0, 10.0, dts)
+    pr.set_medium(med)
+    up = [[x.astype(np.float64) for x in a] for a in (sig, dat)]
+    got = pr.born_forward(sig, pert, spos, rpos)
+    ref = O.born_forward_reg(p, med.astype(np.float64), up[0], pert.astype(np.float64), spos, rpos, np.float64)
+    assert rel_l2(got, ref) < 1e-5
+    got = pr.born_adjoint(sig, dat, spos, rpos)
+    ref = O.born_adjoint_reg(p, med.astype(np.float64), up[0], up[1], spos, rpos, None, np.float64)
+    assert rel_l2(got, ref) < 1e-5
+    pr.close()

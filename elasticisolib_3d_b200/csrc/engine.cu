@@ -560,7 +560,7 @@ static int launchTma(Context* c, const StepPtrs& p, dim3 grid, int yChunk) {
   return E3D_OK;
 }
 
-static int chooseChunks(const Context* c, long long tiles, int nyi, int perSM = 2);
+static int chooseChunks(const Context* c, long long tiles, int nyi, int perSM = 2, int minRun = 24);
 
 // Split stepper: role V maps (stress halos and leads, old velocities, rho planes) and role S maps
 // (velocity halos and leads, old stresses, lambda/mu planes).  shots > 0: the field maps cover
@@ -926,13 +926,13 @@ long long launchCount(const Context* c) { return c->launches; }
 
 // y chunks of a y-marching launch over `tiles` (z, x) tile columns: the CTAs
 // run in waves of perSM per SM, and each CTA pays about two planes of pipeline
-// start-up, so pick the chunk count (y runs of at least 24 planes) that
+// start-up, so pick the chunk count (y runs of at least minRun planes) that
 // minimises waves * (planes per CTA + 2).
-static int chooseChunks(const Context* c, long long tiles, int nyi, int perSM) {
+static int chooseChunks(const Context* c, long long tiles, int nyi, int perSM, int minRun) {
   int chunks = 1;
   const long long slots = (long long)perSM * c->numSMs;
   long long bestCost = -1;
-  for (int ch = 1; ch <= std::max(1, nyi / 24); ch++) {
+  for (int ch = 1; ch <= std::max(1, nyi / minRun); ch++) {
     const long long waves = (tiles * ch + slots - 1) / slots;
     const long long cost = waves * ((nyi + ch - 1) / ch + 2);
     if (bestCost < 0 || cost < bestCost) {
@@ -2207,7 +2207,11 @@ static int launchImagingBlock(Context* c, long long mEnd, float* const v[4], boo
     constexpr size_t smem = (size_t)2 * IMG_STAGE_F * sizeof(float);
     static std::atomic<unsigned long long> configured{0};
     E3D_RET(ensureSmemAttr((const void*)kImagingTma, smem, configured));
-    const int chunks0 = c->imgChunks > 0 ? std::min(c->imgChunks, nyi) : chooseChunks(c, (long long)tiz * tix, nyi);
+    // runs of at least 24 planes where those fill the device, else down to two planes (72x72x64
+    // cells: 16 tiles, 32 CTAs of 28 planes took 74 us, 208 of four take 22)
+    const long long tiles = (long long)tiz * tix;
+    const int minRun = tiles * std::max(1, nyi / 24) >= 2LL * c->numSMs ? 24 : 2;
+    const int chunks0 = c->imgChunks > 0 ? std::min(c->imgChunks, nyi) : chooseChunks(c, tiles, nyi, 2, minRun);
     const int yChunk = (nyi + chunks0 - 1) / chunks0;
     const int chunks = (nyi + yChunk - 1) / yChunk;
     kImagingTma<<<dim3(tiz, tix, chunks), dim3(TZ, IMG_TX), smem, c->st>>>(mp, q, c->g, yChunk);

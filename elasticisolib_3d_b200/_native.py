@@ -61,6 +61,7 @@ SIGNATURES = {
     "e3d_nl_propagate_slabs": ([P, I, I, I] + [P] * 6, I),
     "e3d_born_forward": ([P] * 8, I),
     "e3d_born_adjoint": ([P] * 8, I),
+    "e3d_born_image": ([P] * 8, I),
     "e3d_nl_propagate_device": ([P, I, P, P, P, P, P, P], I),
     "e3d_fwi_forward_device": ([P] * 8, I),
     "e3d_fwi_gradient_device": ([P] * 10, I),

@@ -445,6 +445,14 @@ int e3d_born_adjoint(e3d_context* ctx, const float* const* src9, const float* co
   return bornAdjointHost(ctx->c, src9, data9, geomArrays(src_pos, n_src), geomArrays(rec_pos, n_rec), pert8);
 }
 
+int e3d_born_image(e3d_context* ctx, const float* const* src9, const float* const* data9,
+                   const long long* const* src_pos, const long long* n_src, const long long* const* rec_pos,
+                   const long long* n_rec, float* const* pert8) {
+  CTX_OR_FAIL(ctx);
+  if (!src_pos || !n_src || !rec_pos || !n_rec) return fail(E3D_ERR_ARG, "null geometry");
+  return bornAdjointHost(ctx->c, src9, data9, geomArrays(src_pos, n_src), geomArrays(rec_pos, n_rec), pert8, true);
+}
+
 static int devSet(const long long* pos, const int* off10, DevSignals& s) {
   if (!off10) return fail(E3D_ERR_ARG, "null offsets");
   s.pos = pos;

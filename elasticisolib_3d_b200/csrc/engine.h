@@ -58,8 +58,9 @@ int nlPropagateHost(Context* c, bool adjoint, float* const* model, float* const*
                     const HostGeom& rec);
 int bornForwardHost(Context* c, const float* const* srcSig, float* const* data, const HostGeom& src,
                     const HostGeom& rec, const float* const* pert);
+// fromZero: the image starts at zero, whatever the caller's planes hold (else it adds to them).
 int bornAdjointHost(Context* c, const float* const* srcSig, const float* const* data, const HostGeom& src,
-                    const HostGeom& rec, float* const* pert);
+                    const HostGeom& rec, float* const* pert, bool fromZero = false);
 
 // Device entry points: signals are time-major and concatenated over the nine
 // components ([nts][sum of per-component counts]); positions are device

@@ -344,12 +344,13 @@ class Propagator:
     def born_adjoint(self, src9, data9, src_pos7, rec_pos7, pert8_init=None):
         src = [N.as_f32(s) for s in src9]
         data = [N.as_f32(d) for d in data9]
-        pert = [np.zeros(self.shape, dtype=np.float32) if pert8_init is None else np.array(pert8_init[k],
-                                                                                             dtype=np.float32)
+        # without initial planes the image starts at zero on the device and nothing is sent there
+        fresh = pert8_init is None
+        pert = [np.empty(self.shape, dtype=np.float32) if fresh else np.array(pert8_init[k], dtype=np.float32)
                 for k in range(8)]
         SP, SN, k1 = _geom(src_pos7)
         RP, RN, k2 = _geom(rec_pos7)
-        N.call("e3d_born_adjoint", self._h, N.ptr_array(src), N.ptr_array(data), SP, SN, RP, RN, N.ptr_array(pert))
+        N.call("e3d_born_image" if fresh else "e3d_born_adjoint", self._h, N.ptr_array(src), N.ptr_array(data), SP, SN, RP, RN, N.ptr_array(pert))
         return pert
 
     def kernel_timing(self, every):

@@ -406,6 +406,10 @@ int e3d_born_forward(e3d_context* ctx, const float* const* src9, float* const* d
 int e3d_born_adjoint(e3d_context* ctx, const float* const* src9, const float* const* data9,
                      const long long* const* src_pos, const long long* n_src, const long long* const* rec_pos,
                      const long long* n_rec, float* const* pert8);
+/* e3d_born_adjoint with the image started at zero: pert8 is output only. */
+int e3d_born_image(e3d_context* ctx, const float* const* src9, const float* const* data9,
+                   const long long* const* src_pos, const long long* n_src, const long long* const* rec_pos,
+                   const long long* n_rec, float* const* pert8);
 
 /* Device-buffer propagations.  Signals are time-major [nts][ntot] with the
  * nine components concatenated; pos_dev is the matching int64 table and

@@ -207,6 +207,68 @@ static void fieldFree(Context* c, float* p) {
   if (p) devFree(c, p - c->fieldOff);
 }
 
+// Gives up the padding of the rows where the device has no memory for it: every field buffer is
+// released (they hold nothing between calls; saved checkpoints become invalid) and the medium moves to
+// unpadded rows, plane by plane.
+static int unpadRows(Context* c) {
+  std::vector<float*> old;
+  auto drop = [&](Fields9& f) {
+    for (int k = 0; k < NCOMP; k++) {
+      if (f.p[k] && std::find(old.begin(), old.end(), f.p[k]) == old.end()) old.push_back(f.p[k]);
+      f.p[k] = nullptr;
+    }
+  };
+  for (Fields9* f : {&c->w0, &c->w1, &c->s0, &c->s1, &c->ss[0], &c->ss[1], &c->q0, &c->q1, &c->bw0, &c->bw1}) drop(*f);
+  for (auto* ring : {&c->srcRing, &c->adjRing}) {
+    for (auto& f : *ring) drop(f);
+    ring->clear();
+  }
+  for (float* p : old) fieldFree(c, p);
+  for (float* p : c->vSlots) fieldFree(c, p);
+  for (void* p : c->vStore) devFree(c, p);
+  for (void* p : c->ckpt) devFree(c, p);
+  for (float* p : c->ckptScale) devFree(c, p);
+  c->vSlots.clear();
+  c->vStore.clear();
+  c->ckpt.clear();
+  c->ckptScale.clear();
+  c->batchShots = 0;
+  c->ckptSegLen = 0;
+  c->ckptAllocType = c->vAllocType = -1;
+  c->ckptValid = c->tailValid = false;
+  c->tmaps.clear();
+  // released buffers go back to the device whole, not as holes for the next ones
+  E3D_CUDA_TRY(cudaStreamSynchronize(c->st));
+  cudaMemPool_t pool = nullptr;
+  if (cudaDeviceGetDefaultMemPool(&pool, c->d.device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+  const GridConst g = c->g;
+  const int off = c->fieldOff;
+  c->g.pz = (g.nz + 3) / 4 * 4;
+  c->g.yStride = (long long)c->g.pz * g.nx;
+  c->g.n = c->g.yStride * g.ny;
+  c->fieldOff = FAT;
+  for (int k = 0; k < NMED; k++) {
+    if (!c->med[k]) continue;
+    float* m = nullptr;
+    E3D_RET(fieldAlloc(c, &m));
+    E3D_CUDA_TRY(cudaMemcpy2DAsync(m, (size_t)c->g.pz * sizeof(float), c->med[k], (size_t)g.pz * sizeof(float),
+                                   (size_t)g.nz * sizeof(float), (size_t)g.nx * g.ny, cudaMemcpyDeviceToDevice, c->st));
+    devFree(c, c->med[k] - off);
+    c->med[k] = m;
+  }
+  return E3D_OK;
+}
+
+// Runs a pass that starts from nothing kept, again without the rows' padding if memory ran out.
+template <class Pass>
+static int withRows(Context* c, Pass pass) {
+  int st = pass();
+  if (st != E3D_ERR_OOM || c->fieldOff == FAT) return st;
+  cudaGetLastError();
+  E3D_RET(unpadRows(c));
+  return pass();
+}
+
 static int allocFields(Context* c, Fields9& f, bool zero) {
   const size_t bytes = (size_t)c->g.n * sizeof(float);
   for (int k = 0; k < NCOMP; k++) {
@@ -235,7 +297,8 @@ static int zeroFields(Context* c, Fields9& f, int ncomp = NCOMP) {
 constexpr size_t kStageBytes = (size_t)8 << 20;
 
 static bool staged(Context* c, const void* host, size_t bytes) {
-  if (bytes < kStageBytes / 2) return false;
+  // the buffers cost about 10 ms to pin: only a copy that earns them back makes them
+  if (bytes < (c->stage[1] ? kStageBytes / 2 : 2 * kStageBytes)) return false;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
   else if (at.type != cudaMemoryTypeUnregistered) return false;
@@ -1598,13 +1661,8 @@ int validateDeviceSets(Context* c, const DevSignals& a, const DevSignals& b, int
 // also injects and records over the combined tables, whose positions carry
 // the shot offset.  Loop order of propElasticFwdGpu_3D.
 // ---------------------------------------------------------------------------
-int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const DevSignals& recSet,
-                         const float* srcSig, float* recSig) {
-  E3D_ARG(c && c->haveMedium, "medium not set");
-  E3D_ARG(shots >= 1 && shots <= 1024, "shots must be in [1, 1024]");
-  E3D_ARG(c->d.nz % 4 == 0, "batched propagation needs nz % 4 == 0");
-  E3D_ARG(!c->d.freeSurface, "batched propagation has no free surface");
-  E3D_CUDA_TRY(cudaSetDevice(c->d.device));
+static int nlForwardBatchPass(Context* c, int shots, const DevSignals& srcSet, const DevSignals& recSet,
+                              const float* srcSig, float* recSig) {
   const size_t bytes = (size_t)shots * c->g.n * sizeof(float);
   if (c->batchShots != shots) {
     for (int k = 0; k < NCOMP; k++) {
@@ -1667,10 +1725,18 @@ int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const 
   return flushRecord(c, c->bw1, recSet, true);
 }
 
-int nlPropagateDevice(Context* c, bool adjoint, const DevSignals& srcSet, const DevSignals& recSet, float* srcSig,
-                      float* recSig) {
+int nlForwardBatchDevice(Context* c, int shots, const DevSignals& srcSet, const DevSignals& recSet,
+                         const float* srcSig, float* recSig) {
   E3D_ARG(c && c->haveMedium, "medium not set");
+  E3D_ARG(shots >= 1 && shots <= 1024, "shots must be in [1, 1024]");
+  E3D_ARG(c->d.nz % 4 == 0, "batched propagation needs nz % 4 == 0");
+  E3D_ARG(!c->d.freeSurface, "batched propagation has no free surface");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
+  return withRows(c, [&] { return nlForwardBatchPass(c, shots, srcSet, recSet, srcSig, recSig); });
+}
+
+static int nlPass(Context* c, bool adjoint, const DevSignals& srcSet, const DevSignals& recSet, float* srcSig,
+                  float* recSig) {
   E3D_RET(allocFields(c, c->w0, true));
   E3D_RET(allocFields(c, c->w1, true));
   c->tailReady = takesTail(c);
@@ -1693,6 +1759,13 @@ int nlPropagateDevice(Context* c, bool adjoint, const DevSignals& srcSet, const 
         blocks, first + dir, dir, c->w0, c->w1));
   }
   return flushRecord(c, c->w1, outSet, true);
+}
+
+int nlPropagateDevice(Context* c, bool adjoint, const DevSignals& srcSet, const DevSignals& recSet, float* srcSig,
+                      float* recSig) {
+  E3D_ARG(c && c->haveMedium, "medium not set");
+  E3D_CUDA_TRY(cudaSetDevice(c->d.device));
+  return withRows(c, [&] { return nlPass(c, adjoint, srcSet, recSet, srcSig, recSig); });
 }
 
 int nlPropagateHost(Context* c, bool adjoint, float* const* model, float* const* data, const HostGeom& src,
@@ -2333,7 +2406,13 @@ static int bornForwardDevice(Context* c, const DevSignals& srcSet, const DevSign
   const int nts = c->d.nts, sub = c->d.sub;
   // with a ring of source levels one launch per block decimates them and the steps carry no
   // accumulators (188 -> 140 B per cell and step)
-  const bool ring = ringLevels(c) > 0;
+  bool ring = ringLevels(c) > 0;
+  if (ring && c->srcRing.empty()) {
+    // the ring's levels beside the two kept, if the device has the memory for them and the rest of the pass
+    size_t free = 0, total = 0;
+    E3D_CUDA_TRY(cudaMemGetInfo(&free, &total));
+    ring = 0.9 * (double)free > ((ringLevels(c) + 4.0) * NCOMP + 12.0) * sizeof(float) * c->g.n;
+  }
   if (ring) {
     E3D_RET(ensureRing(c, c->srcRing, c->s0, c->s1, ringLevels(c)));
   } else {
@@ -3155,7 +3234,7 @@ int bornForwardHost(Context* c, const float* const* srcSig, float* const* data, 
   if (st == E3D_OK) st = stageGeom(c, rec, true, R);
   if (st == E3D_OK) st = stageSignalsIn(c, S, srcSig);
   if (st == E3D_OK) st = stageSignalsZero(c, R);
-  if (st == E3D_OK) st = bornForwardDevice(c, S.set, R.set, S.sig, R.sig);
+  if (st == E3D_OK) st = withRows(c, [&] { return bornForwardDevice(c, S.set, R.set, S.sig, R.sig); });
   if (st == E3D_OK) st = stageSignalsOut(c, R, data);
   if (st == E3D_OK) st = checkPipeError(c);
   if (st == E3D_OK && cudaStreamSynchronize(c->st) != cudaSuccess) {
@@ -3187,7 +3266,7 @@ int bornAdjointHost(Context* c, const float* const* srcSig, const float* const* 
   if (st == E3D_OK) st = stageGeom(c, rec, true, R);
   if (st == E3D_OK) st = stageSignalsIn(c, S, srcSig);
   if (st == E3D_OK) st = stageSignalsIn(c, R, const_cast<float* const*>(data));
-  if (st == E3D_OK) st = bornAdjointDevice(c, S.set, R.set, S.sig, R.sig);
+  if (st == E3D_OK) st = withRows(c, [&] { return bornAdjointDevice(c, S.set, R.set, S.sig, R.sig); });
   if (st == E3D_OK) st = checkPipeError(c);
   if (st == E3D_OK) {
     for (int k = 0; k < NMED && st == E3D_OK; k++) st = copyOut(c, pert[k], c->pertDev[k], planeBytes);
@@ -3208,7 +3287,7 @@ int fwiForwardDevice(Context* c, const DevSignals& srcSet, const DevSignals& rec
   E3D_ARG(c->d.nts >= 2, "FWI needs at least two coarse samples");
   E3D_RET(rejectFreeSurface(c));
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
-  return sourcePassWithCheckpoints(c, srcSet, &recSet, srcSig, recSig, map);
+  return withRows(c, [&] { return sourcePassWithCheckpoints(c, srcSet, &recSet, srcSig, recSig, map); });
 }
 
 int fwiGradientDevice(Context* c, const DevSignals& srcSet, const DevSignals& recSet, const float* srcSig,

@@ -99,3 +99,33 @@ def test_born_pair_matches_oracle(nz, nx, ny, nts, sub, nsrc, nrec):
     ref = O.born_adjoint_reg(p, med.astype(np.float64), up[0], up[1], spos, rpos, None, np.float64)
     assert rel_l2(got, ref) < 1e-5
     pr.close()
+
+
+def test_padded_rows_give_way_to_memory():
+    """A batch that fits the device in unpadded rows only (72-cell rows: a third more when padded) runs,
+    with the traces of one that had the room."""
+    import torch
+    nz, nx, ny, nts, sub, shots = 72, 200, 200, 4, 4, 10
+    rng = np.random.default_rng(3)
+    el = S.elastic_from_velocity(*S.gaussian_perturbed_model((ny, nx, nz), 2500.0, 1443.0, 2000.0, 0.1, 2.0, 5))
+    med = O.medium_planes(el, 0.0005, np.float32)
+    spos = [[_points(rng, nz, nx, ny, 5) for _ in range(7)] for _ in range(shots)]
+    rpos = [_points(rng, nz, nx, ny, 300) for _ in range(7)]
+    models = [random_signals(sp, nts, rng) for sp in spos]
+    out = []
+    for full in (False, True):
+        pr = Propagator(nz, nx, ny, nts, sub, 8, 10.0, 10.0, 10.0, 0.002, q2compat=0)
+        pr.set_medium(med)
+        torch.cuda.empty_cache()
+        hog = None
+        if full:
+            free, _ = torch.cuda.mem_get_info()
+            hog = torch.empty(int(free - 18 * 4 * nz * nx * ny * shots * 1.15 - (64 << 20)), dtype=torch.uint8,
+                              device="cuda")
+        out.append(pr.nl_forward_batch(models, spos, rpos))
+        pr.close()
+        del hog
+        torch.cuda.empty_cache()
+    for a, b in zip(*out):
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)

@@ -289,7 +289,7 @@ static int zeroFields(Context* c, Fields9& f, int ncomp = NCOMP) {
 
 // ---------------------------------------------------------------------------
 // Copies of whole planes between the device and the caller's pageable memory.  The driver stages
-// those on one host thread: measured on the B200 box at 141 MB, 12 GB/s in and 4 to 6 GB/s out, where
+// those on one host thread: measured beside a B200 at 141 MB, 12 GB/s in and 4 to 6 GB/s out, where
 // every page of a fresh array is also touched for the first time.  Here two pinned buffers
 // alternate between the bus and a memcpy over several host threads.  Small copies and callers' pinned
 // memory go straight to cudaMemcpyAsync.

@@ -799,30 +799,19 @@ static bool pairPath(const Context* c, int mode, const StepPtrs& p) {
 // of `tail`.  Plain launches: programmatic ones (the next step's CTAs waiting in freed slots) measured
 // slower on B200, 108.7 against 103.4 us a step at 168x152x171 cells and 12.3 against 10.5 at 72x72x60
 // with 8-plane runs, because the early CTAs take their slots unevenly.
-template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE, int U>
-static int launchPairU(Context* c, const StepPtrs& p, const StepTail& tail, int shots) {
+template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE>
+static int launchPair(Context* c, const StepPtrs& p, const StepTail& tail, int shots) {
   constexpr size_t smem = (size_t)STAGES * SPL_STAGE_F * sizeof(float);
   static std::atomic<unsigned long long> configured{0};
-  E3D_RET(ensureSmemAttr((const void*)kStepSplitPair<MODE, STAGES, MINB, BATCH, SS, EDGE, U>, smem, configured));
+  E3D_RET(ensureSmemAttr((const void*)kStepSplitPair<MODE, STAGES, MINB, BATCH, SS, EDGE>, smem, configured));
   SplitMaps mp;
   E3D_RET(buildSplitMaps(c, p, mp, BATCH ? shots : 0));
   const PairShape s = pairShape(c, shots);
-  kStepSplitPair<MODE, STAGES, MINB, BATCH, SS, EDGE, U>
+  kStepSplitPair<MODE, STAGES, MINB, BATCH, SS, EDGE>
       <<<dim3(s.tilesZ * shots, s.tilesX, 2 * s.chunks + tail.recBlocks), dim3(TZ / 2, 8), smem, c->st>>>(
           mp, p, c->g, s.yChunk, s.chunks, shots, tail);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
-}
-
-// Two planes a pass from four waves of CTAs on (kStepSplitPair says what each costs).
-template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE>
-static int launchPair(Context* c, const StepPtrs& p, const StepTail& tail, int shots) {
-  if (STAGES == 3 && !EDGE) {
-    const PairShape s = pairShape(c, shots);
-    if (2LL * s.tilesZ * shots * s.tilesX * s.chunks >= 4LL * MINB * c->numSMs)
-      return launchPairU<MODE, STAGES, MINB, BATCH, SS, EDGE, STAGES == 3 && !EDGE ? 2 : 1>(c, p, tail, shots);
-  }
-  return launchPairU<MODE, STAGES, MINB, BATCH, SS, EDGE, 1>(c, p, tail, shots);
 }
 
 template <int MODE>

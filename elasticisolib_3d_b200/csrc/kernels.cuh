@@ -883,10 +883,7 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
 // memory as 8-byte pairs: a z derivative of both cells takes 5 paired loads
 // instead of 16 single ones, an x derivative 8 instead of 16, and the old level,
 // medium and y-window planes one paired load per field; the new level is
-// stored as float2.  Along x and y, and in the update, both cells' arithmetic runs in two-wide FP32
-// instructions, each half rounded as kStepSplit rounds it (measured against scalar ones on B200:
-// 72x72x60 cells 8.8 -> 8.3 us a step, 104x104x96 22.3 -> 21.4, 392x392x388 1557 -> 1530 under the
-// power cap, where fewer instructions leave a higher clock).
+// stored as float2.  Each cell's arithmetic is kStepSplit's, term by term.
 // blockDim (TZ/2, 8); forward and time-reversed modes.  The launch also does
 // what surrounds the step: the free surface's images, a Born secondary source,
 // the injection of few points and the recording of the level before (StepTail).
@@ -894,62 +891,28 @@ __device__ __forceinline__ void splitRole(const CUtensorMap* mp, const StepPtrs&
 __device__ __forceinline__ float2 lds2(const float* t, int i) { return *reinterpret_cast<const float2*>(t + i); }
 
 // z derivatives of cells i and i+1 (i even) of a shared tile row: forward (+) and backward (-)
-__device__ __forceinline__ float2 dPlusZ2(const float* t, int i, const float* c) {
-  float r0, r1;
+__device__ __forceinline__ void dPlusZ2(const float* t, int i, const float* c, float& r0, float& r1) {
   const float2 a = lds2(t, i - 4), b = lds2(t, i - 2), m = lds2(t, i), d = lds2(t, i + 2), e = lds2(t, i + 4);
   r0 = c[0] * (m.y - m.x) + c[1] * (d.x - b.y) + c[2] * (d.y - b.x) + c[3] * (e.x - a.y);
   r1 = c[0] * (d.x - m.y) + c[1] * (d.y - m.x) + c[2] * (e.x - b.y) + c[3] * (e.y - b.x);
-  return make_float2(r0, r1);
 }
-__device__ __forceinline__ float2 dMinusZ2(const float* t, int i, const float* c) {
-  float r0, r1;
+__device__ __forceinline__ void dMinusZ2(const float* t, int i, const float* c, float& r0, float& r1) {
   const float2 a = lds2(t, i - 4), b = lds2(t, i - 2), m = lds2(t, i), d = lds2(t, i + 2), e = lds2(t, i + 4);
   r0 = c[0] * (m.x - b.y) + c[1] * (m.y - b.x) + c[2] * (d.x - a.y) + c[3] * (d.y - a.x);
   r1 = c[0] * (m.y - m.x) + c[1] * (d.x - b.y) + c[2] * (d.y - b.x) + c[3] * (e.x - a.y);
-  return make_float2(r0, r1);
-}
-// Two cells' FP32 arithmetic in one instruction (each half rounded as the scalar one).
-__device__ __forceinline__ unsigned long long bits2(float2 a) {
-  return (unsigned long long)__float_as_uint(a.y) << 32 | __float_as_uint(a.x);
-}
-__device__ __forceinline__ float2 from2(unsigned long long v) {
-  return make_float2(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
-  return from2(r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)));
-  return from2(r);
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
-  return from2(r);
-}
-__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, both(-1.0f), a); }  // a - b, rounded once
-
-// c[0] (a - b) + c[1] (e - f) + c[2] (g - h) + c[3] (k - l) of two cells
-__device__ __forceinline__ float2 stencil2(float2 a, float2 b, float2 e, float2 f, float2 g, float2 h, float2 k,
-                                           float2 l, const float* c) {
-  return fma2(both(c[3]), sub2(k, l), fma2(both(c[2]), sub2(g, h), fma2(both(c[1]), sub2(e, f), mul2(both(c[0]), sub2(a, b)))));
 }
 // derivatives of cells i and i+1 along the tile's x axis (stride s, even)
-__device__ __forceinline__ float2 dPlusX2(const float* t, int i, int s, const float* c) {
-  return stencil2(lds2(t, i + s), lds2(t, i), lds2(t, i + 2 * s), lds2(t, i - s), lds2(t, i + 3 * s),
-                  lds2(t, i - 2 * s), lds2(t, i + 4 * s), lds2(t, i - 3 * s), c);
+__device__ __forceinline__ void dPlusX2(const float* t, int i, int s, const float* c, float& r0, float& r1) {
+  const float2 m3 = lds2(t, i - 3 * s), m2 = lds2(t, i - 2 * s), m1 = lds2(t, i - s), p0 = lds2(t, i);
+  const float2 p1 = lds2(t, i + s), p2 = lds2(t, i + 2 * s), p3 = lds2(t, i + 3 * s), p4 = lds2(t, i + 4 * s);
+  r0 = c[0] * (p1.x - p0.x) + c[1] * (p2.x - m1.x) + c[2] * (p3.x - m2.x) + c[3] * (p4.x - m3.x);
+  r1 = c[0] * (p1.y - p0.y) + c[1] * (p2.y - m1.y) + c[2] * (p3.y - m2.y) + c[3] * (p4.y - m3.y);
 }
-__device__ __forceinline__ float2 dMinusX2(const float* t, int i, int s, const float* c) {
-  return stencil2(lds2(t, i), lds2(t, i - s), lds2(t, i + s), lds2(t, i - 2 * s), lds2(t, i + 2 * s),
-                  lds2(t, i - 3 * s), lds2(t, i + 3 * s), lds2(t, i - 4 * s), c);
-}
-// along y, from the window of planes
-__device__ __forceinline__ float2 dWin2(const float2* w, const float* c) {
-  return stencil2(w[4], w[3], w[5], w[2], w[6], w[1], w[7], w[0], c);
+__device__ __forceinline__ void dMinusX2(const float* t, int i, int s, const float* c, float& r0, float& r1) {
+  const float2 m4 = lds2(t, i - 4 * s), m3 = lds2(t, i - 3 * s), m2 = lds2(t, i - 2 * s), m1 = lds2(t, i - s);
+  const float2 p0 = lds2(t, i), p1 = lds2(t, i + s), p2 = lds2(t, i + 2 * s), p3 = lds2(t, i + 3 * s);
+  r0 = c[0] * (p0.x - m1.x) + c[1] * (p1.x - m2.x) + c[2] * (p2.x - m3.x) + c[3] * (p3.x - m4.x);
+  r1 = c[0] * (p0.y - m1.y) + c[1] * (p1.y - m2.y) + c[2] * (p2.y - m3.y) + c[3] * (p3.y - m4.y);
 }
 
 // What a paired stepper launch does beside the step itself.
@@ -1113,14 +1076,9 @@ __device__ __forceinline__ void stepRecord(const StepTail& t, const GridConst& g
 // BATCH: nshots shots stacked per field (shot s at offset s*n), 4D field maps, blockIdx.x = tile *
 // nshots + shot: consecutive CTAs take one tile for consecutive shots, so a medium tile fetched for
 // one shot is in L2 for the others.
-// U planes a pass over the body: the y-windows move U planes at once, so U = 2 halves their register
-// moves; its twice longer body starts slower, which short launches feel.  Measured on B200, one against
-// two planes: 392x392x388 cells 1569 -> 1482 us a step under the power cap (1440 -> 1380 before it acts),
-// 168x200x188 139.9 -> 138.4, but 104x104x96 21.4 -> 23.6, 72x72x60 8.4 -> 9.9; four planes are slower
-// everywhere.
 // EDGE: rows of an odd number of cells or a free surface (tail.surface); the common form carries
 // neither's branches (measured on B200 at 72x72x60 cells, 4-plane runs: 8.9 against 9.5 us a step).
-template <int MODE, bool ROLE_S, int STAGES, bool BATCH, bool SS, bool EDGE, int U>
+template <int MODE, bool ROLE_S, int STAGES, bool BATCH, bool SS, bool EDGE>
 __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepPtrs& p, const GridConst& g,
                                               int yChunk, int chunk, float* smem, unsigned long long* bars,
                                               int nshots, const StepTail& tail) {
@@ -1157,13 +1115,16 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
       if (yBeg + s < yEnd)
         splitIssuePlane<ROLE_S, BATCH>(mp, smem + s * SPL_STAGE_F, &bars[s], yBeg + s, z0, x0, shot);
   }
-  float2 w[3][7 + U];  // y-windows of cells iz and iz+1; plane u of a pass over the body starts at w[.][u]
+  float w0[3][8], w1[3][8];  // y-windows of cells iz and iz+1
   if (active) {
 #pragma unroll
     for (int q = 0; q < 3; q++)
 #pragma unroll
-      for (int k = 0; k < 7; k++)
-        w[q][k] = __ldg(reinterpret_cast<const float2*>(p.c[R::lead(q)] + (long long)(yBeg + R::base(q) + k) * ys + col));
+      for (int k = 0; k < 7; k++) {
+        const float2 v = __ldg(reinterpret_cast<const float2*>(p.c[R::lead(q)] + (long long)(yBeg + R::base(q) + k) * ys + col));
+        w0[q][k] = v.x;
+        w1[q][k] = v.y;
+      }
   }
   int dzx[2];
   float Gzx[2];
@@ -1180,122 +1141,168 @@ __device__ __forceinline__ void splitRolePair(const CUtensorMap* mp, const StepP
   for (int k = 0; k < R::NO; k++) out[k] = (p.nw[0] ? p.nw[R::C0 + k] : p.o[R::C0 + k]) + col;
   int slot = 0;
   unsigned parity = 0;
-  for (int yy = yBeg; yy < yEnd; yy += U) {
+  for (int y = yBeg; y < yEnd; y++) {
+    const int dyy = yDistance(g, y);
+    const float Gy = dyy < g.minPad ? __ldg(g.taper + dyy) : 1.0f;
+    const long long iy = (long long)y * ys;
+    float2 sL[SS ? R::NO : 1], sR[SS ? R::NO : 1];
+    if (SS && active) {
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int y = yy + u;
-      if (u && y >= yEnd) break;
-      const int dyy = yDistance(g, y);
-      const float Gy = dyy < g.minPad ? __ldg(g.taper + dyy) : 1.0f;
-      const long long iy = (long long)y * ys;
-      float2 sL[SS ? R::NO : 1], sR[SS ? R::NO : 1];
-      if (SS && active) {
-#pragma unroll
-        for (int k = 0; k < R::NO; k++) {
-          sL[k] = __ldg(reinterpret_cast<const float2*>(p.ssL[R::C0 + k] + col + iy));
-          sR[k] = __ldg(reinterpret_cast<const float2*>(p.ssR[R::C0 + k] + col + iy));
-        }
+      for (int k = 0; k < R::NO; k++) {
+        sL[k] = __ldg(reinterpret_cast<const float2*>(p.ssL[R::C0 + k] + col + iy));
+        sR[k] = __ldg(reinterpret_cast<const float2*>(p.ssR[R::C0 + k] + col + iy));
       }
-      const bool ok = mbarWaitBounded(&bars[slot], (parity >> slot) & 1u);
-      if (__syncthreads_or(!ok)) {
-        if (tid == 0) {
-          atomicExch(&g_e3dPipeError, 1u);
-          for (int s = 0; s < STAGES; s++) mbarWaitBounded(&bars[s], (parity >> s) & 1u);
-        }
-        __syncthreads();
-        return;
-      }
-      parity ^= 1u << slot;
+    }
+    const bool ok = mbarWaitBounded(&bars[slot], (parity >> slot) & 1u);
+    if (__syncthreads_or(!ok)) {
       if (tid == 0) {
-        const int yn = y + STAGES - 1;
-        int ns = slot + STAGES - 1;
-        if (ns >= STAGES) ns -= STAGES;
-        if (yn < yEnd) splitIssuePlane<ROLE_S, BATCH>(mp, smem + ns * SPL_STAGE_F, &bars[ns], yn, z0, x0, shot);
+        atomicExch(&g_e3dPipeError, 1u);
+        for (int s = 0; s < STAGES; s++) mbarWaitBounded(&bars[s], (parity >> s) & 1u);
       }
-      const float* st = smem + slot * SPL_STAGE_F;
-      if (active) {
+      __syncthreads();
+      return;
+    }
+    parity ^= 1u << slot;
+    if (tid == 0) {
+      const int yn = y + STAGES - 1;
+      int ns = slot + STAGES - 1;
+      if (ns >= STAGES) ns -= STAGES;
+      if (yn < yEnd) splitIssuePlane<ROLE_S, BATCH>(mp, smem + ns * SPL_STAGE_F, &bars[ns], yn, z0, x0, shot);
+    }
+    const float* st = smem + slot * SPL_STAGE_F;
+    if (active) {
 #pragma unroll
-        for (int q = 0; q < 3; q++) w[q][7 + u] = lds2(st, R::LEAD_OFF + q * SPL_INT_F + li);
-        const float* cz = g.cz;
-        const float* cx = g.cx;
-        const float* cy = g.cy;
-        const float2 G = make_float2(dyy < dzx[0] ? Gy : Gzx[0], dyy < dzx[1] ? Gy : Gzx[1]);
-        const float2 sgn = both((MODE == STEP_FWD) ? 1.0f : -1.0f);
-        // the new level: G (G old + sgn up [+ the secondary source])
-        auto update = [&](int k, float2 up) {
-          float2 u = fma2(G, lds2(st, R::OLD_OFF + k * SPL_INT_F + li), MODE == STEP_FWD ? up : mul2(sgn, up));
-          if (SS) u = fma2(sL[k], both(p.ssWl), fma2(sR[k], both(p.ssWr), u));
-          return mul2(G, u);
-        };
-        auto medium = [&](int k) { return lds2(st, R::MED_OFF + k * SPL_INT_F + li); };
-        float2 nv[R::NO];
-        if (!ROLE_S) {
-          const float* tSXX = st;
-          const float* tSXY = st + SPL_HALO_F;
-          const float* tSXZ = st + 2 * SPL_HALO_F;
-          const float* tSYZ = st + 3 * SPL_HALO_F;
-          const float* tSZZ = st + 4 * SPL_HALO_F;
-          const float2 fx = add2(add2(dMinusX2(tSXX, lc, SZ, cx), dWin2(w[0] + u, cy)), dPlusZ2(tSXZ, lc, cz));
-          const float2 fy = add2(add2(dPlusX2(tSXY, lc, SZ, cx), dWin2(w[1] + u, cy)), dPlusZ2(tSYZ, lc, cz));
-          const float2 fz = add2(add2(dPlusX2(tSXZ, lc, SZ, cx), dWin2(w[2] + u, cy)), dMinusZ2(tSZZ, lc, cz));
-          nv[0] = update(0, mul2(medium(0), fx));
-          nv[1] = update(1, mul2(medium(1), fy));
-          nv[2] = update(2, mul2(medium(2), fz));
-          if (EDGE && tail.surface && iz == FAT) nv[VZ].x = 0.0f;  // the ghost row half a cell above the surface
-        } else {
-          const float* tVX = st;
-          const float* tVY = st + SPL_HALO_F;
-          const float* tVZ = st + 2 * SPL_HALO_F;
-          const float2 dxx = dPlusX2(tVX, lc, SZ, cx), dyy2 = dWin2(w[1] + u, cy), dzz = dPlusZ2(tVZ, lc, cz);
-          const float2 fxy = add2(dWin2(w[0] + u, cy), dMinusX2(tVY, lc, SZ, cx));
-          const float2 fxz = add2(dMinusZ2(tVX, lc, cz), dMinusX2(tVZ, lc, SZ, cx));
-          const float2 fyz = add2(dWin2(w[2] + u, cy), dMinusZ2(tVY, lc, cz));
-          const float2 l2m = medium(0), lam = medium(1);
-          nv[0] = update(0, fma2(l2m, dxx, mul2(lam, add2(dyy2, dzz))));
-          nv[1] = update(1, fma2(l2m, dyy2, mul2(lam, add2(dxx, dzz))));
-          nv[2] = update(2, fma2(l2m, dzz, mul2(lam, add2(dxx, dyy2))));
-          nv[3] = update(3, mul2(medium(2), fxz));
-          nv[4] = update(4, mul2(medium(3), fxy));
-          nv[5] = update(5, mul2(medium(4), fyz));
-          if (EDGE && tail.surface && iz <= 2 * FAT) {
-            // stress imaging about the surface row FAT (the conditions kFreeSurface states), each row
-            // writing its image: szz rows FAT+1..2 FAT, sxz and syz rows FAT+1..2 FAT+1
-            if (iz == FAT) {
-              const float corr = sgn.x * G.x * (-lam.x * dzz.x - (lam.x * lam.x / l2m.x) * (dxx.x + dyy2.x));
-              nv[0].x += corr;
-              nv[1].x += corr;
-              nv[2].x = 0.0f;
-              nv[3].x = -nv[3].y;
-              nv[5].x = -nv[5].y;
-              out[2][iy - 1] = -nv[2].y;
-            } else {
-              const int up2 = 2 * (iz - FAT);
-              out[2][iy - up2] = -nv[2].x;
-              if (iz < 2 * FAT) out[2][iy - up2 - 1] = -nv[2].y;
-              out[3][iy - up2 + 1] = -nv[3].x;
-              out[3][iy - up2] = -nv[3].y;
-              out[5][iy - up2 + 1] = -nv[5].x;
-              out[5][iy - up2] = -nv[5].y;
-            }
+      for (int q = 0; q < 3; q++) {
+        const float2 v = lds2(st, R::LEAD_OFF + q * SPL_INT_F + li);
+        w0[q][7] = v.x;
+        w1[q][7] = v.y;
+      }
+      const float* cz = g.cz;
+      const float* cx = g.cx;
+      const float* cy = g.cy;
+      const float G[2] = {dyy < dzx[0] ? Gy : Gzx[0], dyy < dzx[1] ? Gy : Gzx[1]};
+      const float sgn = (MODE == STEP_FWD) ? 1.0f : -1.0f;
+      float2 nv[R::NO];
+      if (!ROLE_S) {
+        const float* tSXX = st;
+        const float* tSXY = st + SPL_HALO_F;
+        const float* tSXZ = st + 2 * SPL_HALO_F;
+        const float* tSYZ = st + 3 * SPL_HALO_F;
+        const float* tSZZ = st + 4 * SPL_HALO_F;
+        float a0, a1, b0, b1, e0, e1;
+        float fv[3][2];
+        dMinusX2(tSXX, lc, SZ, cx, a0, a1);
+        dPlusZ2(tSXZ, lc, cz, b0, b1);
+        fv[0][0] = a0 + dWin(w0[0], cy) + b0;
+        fv[0][1] = a1 + dWin(w1[0], cy) + b1;
+        dPlusX2(tSXY, lc, SZ, cx, a0, a1);
+        dPlusZ2(tSYZ, lc, cz, b0, b1);
+        fv[1][0] = a0 + dWin(w0[1], cy) + b0;
+        fv[1][1] = a1 + dWin(w1[1], cy) + b1;
+        dPlusX2(tSXZ, lc, SZ, cx, a0, a1);
+        dMinusZ2(tSZZ, lc, cz, e0, e1);
+        fv[2][0] = a0 + dWin(w0[2], cy) + e0;
+        fv[2][1] = a1 + dWin(w1[2], cy) + e1;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+          const float2 rho = lds2(st, R::MED_OFF + k * SPL_INT_F + li);
+          const float2 ov = lds2(st, R::OLD_OFF + k * SPL_INT_F + li);
+          float ux = G[0] * ov.x + sgn * (rho.x * fv[k][0]);
+          float uy = G[1] * ov.y + sgn * (rho.y * fv[k][1]);
+          if (SS) {
+            ux += sL[k].x * p.ssWl + sR[k].x * p.ssWr;
+            uy += sL[k].y * p.ssWl + sR[k].y * p.ssWr;
+          }
+          nv[k] = make_float2(G[0] * ux, G[1] * uy);
+        }
+        if (EDGE && tail.surface && iz == FAT) nv[VZ].x = 0.0f;  // the ghost row half a cell above the surface
+      } else {
+        const float* tVX = st;
+        const float* tVY = st + SPL_HALO_F;
+        const float* tVZ = st + 2 * SPL_HALO_F;
+        float dxx[2], dyy_[2], dzz[2], fxy[2], fxz[2], fyz[2], a0, a1, b0, b1;
+        dPlusX2(tVX, lc, SZ, cx, dxx[0], dxx[1]);
+        dyy_[0] = dWin(w0[1], cy);
+        dyy_[1] = dWin(w1[1], cy);
+        dPlusZ2(tVZ, lc, cz, dzz[0], dzz[1]);
+        dMinusX2(tVY, lc, SZ, cx, a0, a1);
+        fxy[0] = dWin(w0[0], cy) + a0;
+        fxy[1] = dWin(w1[0], cy) + a1;
+        dMinusZ2(tVX, lc, cz, a0, a1);
+        dMinusX2(tVZ, lc, SZ, cx, b0, b1);
+        fxz[0] = a0 + b0;
+        fxz[1] = a1 + b1;
+        dMinusZ2(tVY, lc, cz, a0, a1);
+        fyz[0] = dWin(w0[2], cy) + a0;
+        fyz[1] = dWin(w1[2], cy) + a1;
+        const float2 l2m = lds2(st, R::MED_OFF + li), lam = lds2(st, R::MED_OFF + SPL_INT_F + li);
+        const float2 muxz = lds2(st, R::MED_OFF + 2 * SPL_INT_F + li);
+        const float2 muxy = lds2(st, R::MED_OFF + 3 * SPL_INT_F + li);
+        const float2 muyz = lds2(st, R::MED_OFF + 4 * SPL_INT_F + li);
+        const float L2M_[2] = {l2m.x, l2m.y}, LAM_[2] = {lam.x, lam.y};
+        const float MXZ[2] = {muxz.x, muxz.y}, MXY[2] = {muxy.x, muxy.y}, MYZ[2] = {muyz.x, muyz.y};
+        float up[6][2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          up[0][h] = sgn * (L2M_[h] * dxx[h] + LAM_[h] * (dyy_[h] + dzz[h]));
+          up[1][h] = sgn * (L2M_[h] * dyy_[h] + LAM_[h] * (dxx[h] + dzz[h]));
+          up[2][h] = sgn * (L2M_[h] * dzz[h] + LAM_[h] * (dxx[h] + dyy_[h]));
+          up[3][h] = sgn * (MXZ[h] * fxz[h]);
+          up[4][h] = sgn * (MXY[h] * fxy[h]);
+          up[5][h] = sgn * (MYZ[h] * fyz[h]);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+          const float2 ov = lds2(st, R::OLD_OFF + k * SPL_INT_F + li);
+          float ux = G[0] * ov.x + up[k][0];
+          float uy = G[1] * ov.y + up[k][1];
+          if (SS) {
+            ux += sL[k].x * p.ssWl + sR[k].x * p.ssWr;
+            uy += sL[k].y * p.ssWl + sR[k].y * p.ssWr;
+          }
+          nv[k] = make_float2(G[0] * ux, G[1] * uy);
+        }
+        if (EDGE && tail.surface && iz <= 2 * FAT) {
+          // stress imaging about the surface row FAT (the conditions kFreeSurface states), each row
+          // writing its image: szz rows FAT+1..2 FAT, sxz and syz rows FAT+1..2 FAT+1
+          if (iz == FAT) {
+            const float corr = sgn * G[0] * (-LAM_[0] * dzz[0] - (LAM_[0] * LAM_[0] / L2M_[0]) * (dxx[0] + dyy_[0]));
+            nv[0].x += corr;
+            nv[1].x += corr;
+            nv[2].x = 0.0f;
+            nv[3].x = -nv[3].y;
+            nv[5].x = -nv[5].y;
+            out[2][iy - 1] = -nv[2].y;
+          } else {
+            const int up2 = 2 * (iz - FAT);
+            out[2][iy - up2] = -nv[2].x;
+            if (iz < 2 * FAT) out[2][iy - up2 - 1] = -nv[2].y;
+            out[3][iy - up2 + 1] = -nv[3].x;
+            out[3][iy - up2] = -nv[3].y;
+            out[5][iy - up2 + 1] = -nv[5].x;
+            out[5][iy - up2] = -nv[5].y;
           }
         }
-#pragma unroll
-        for (int k = 0; k < R::NO; k++) {
-          if (pair) *reinterpret_cast<float2*>(out[k] + iy) = nv[k];
-          else out[k][iy] = nv[k].x;
-        }
       }
-      slot = (slot + 1 == STAGES) ? 0 : slot + 1;
+#pragma unroll
+      for (int k = 0; k < R::NO; k++) {
+        if (pair) *reinterpret_cast<float2*>(out[k] + iy) = nv[k];
+        else out[k][iy] = nv[k].x;
+      }
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+#pragma unroll
+        for (int k = 0; k < 7; k++) {
+          w0[q][k] = w0[q][k + 1];
+          w1[q][k] = w1[q][k + 1];
+        }
     }
-#pragma unroll
-    for (int q = 0; q < 3; q++)
-#pragma unroll
-      for (int k = 0; k < 7; k++) w[q][k] = w[q][k + U];
+    slot = (slot + 1 == STAGES) ? 0 : slot + 1;
   }
   if (i0 < i1) stepInject<ROLE_S, NT>(tail, g, dst, p.m, tid, i0, i1);
 }
 
-template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE, int U>
+template <int MODE, int STAGES, int MINB, bool BATCH, bool SS, bool EDGE>
 __global__ void __launch_bounds__(TZ / 2 * 8, MINB) kStepSplitPair(const __grid_constant__ SplitMaps mp,
                                                                    const __grid_constant__ StepPtrs p,
                                                                    const __grid_constant__ GridConst g, int yChunk,
@@ -1304,12 +1311,12 @@ __global__ void __launch_bounds__(TZ / 2 * 8, MINB) kStepSplitPair(const __grid_
   extern __shared__ __align__(1024) float smem[];
   __shared__ __align__(8) unsigned long long bars[STAGES];
   if ((int)blockIdx.z < chunksV)
-    splitRolePair<MODE, false, STAGES, BATCH, SS, EDGE, U>(mp.v, p, g, yChunk, blockIdx.z, smem, bars, nshots, tail);
+    splitRolePair<MODE, false, STAGES, BATCH, SS, EDGE>(mp.v, p, g, yChunk, blockIdx.z, smem, bars, nshots, tail);
   else if ((int)blockIdx.z >= 2 * chunksV)
     stepRecord<TZ / 2 * 8>(tail, g, p.c, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * (blockIdx.z - 2 * chunksV)),
                            threadIdx.y * (TZ / 2) + threadIdx.x);
   else
-    splitRolePair<MODE, true, STAGES, BATCH, SS, EDGE, U>(mp.s, p, g, yChunk, blockIdx.z - chunksV, smem, bars, nshots, tail);
+    splitRolePair<MODE, true, STAGES, BATCH, SS, EDGE>(mp.s, p, g, yChunk, blockIdx.z - chunksV, smem, bars, nshots, tail);
 }
 
 // Owner tables of the acquisition points (AcqEntry): the CTA that updates the component at the cell.

@@ -55,27 +55,6 @@ def test_paired_step_matches_oracle(nz, nx, ny, nts, sub, nsrc, nrec, adjoint, s
     pr.close()
 
 
-@pytest.mark.parametrize("chunks", [17, 25, 0])
-def test_two_planes_a_pass_match_oracle(chunks):
-    """Launches of at least four waves take two planes a pass: y runs of three planes (the last of one),
-    of two, and the automatic ones, against one FP64 oracle run (the same 1e-5)."""
-    nz, nx, ny, nts, sub = 136, 136, 57, 5, 4
-    rng = np.random.default_rng(7)
-    el = S.elastic_from_velocity(*S.gaussian_perturbed_model((ny, nx, nz), 2500.0, 1443.0, 2000.0, 0.1, 4.0, 5))
-    med = O.medium_planes(el, 0.0005, np.float32)
-    p = O.PropParams(nz, nx, ny, nts, sub, 8, 10.0, 10.0, 10.0, 0.002)
-    spos = [_points(rng, nz, nx, ny, 500) for _ in range(7)]
-    rpos = [_points(rng, nz, nx, ny, 2000) for _ in range(7)]
-    sig = random_signals(spos, nts, rng)
-    pr = Propagator(nz, nx, ny, nts, sub, 8, 10.0, 10.0, 10.0, 0.002)
-    pr.set_medium(med)
-    pr.set_stepper_chunks(chunks)
-    got = pr.nl_forward(sig, spos, rpos)
-    ref = O.nl_forward_reg(p, med.astype(np.float64), [s.astype(np.float64) for s in sig], spos, rpos, np.float64)
-    assert rel_l2(got, ref) < 1e-5
-    pr.close()
-
-
 @pytest.mark.parametrize("nz,nx,ny,nts,sub,nsrc,nrec", GRIDS)
 def test_born_pair_matches_oracle(nz, nx, ny, nts, sub, nsrc, nrec):
     """The linearised pair on the same grids: secondary sources in the paired step, source levels

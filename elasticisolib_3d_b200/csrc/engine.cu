@@ -109,6 +109,7 @@ struct Context {
   std::vector<void*> owned;  // every device allocation of this context
   // working wavefields (primary propagation)
   Fields9 w0, w1;
+  bool ghosts = false;       // a slab run left its neighbours' planes in the FAT planes of w0 and w1
   // Born / FWI buffers, allocated on first use
   Fields9 s0, s1;            // source-side state
   std::vector<float*> vSlots;  // decimated source velocity slots, FP32 (3 fields each)
@@ -1948,6 +1949,7 @@ int nlPropagateSlabsHost(Context* const* slabs, int nSlabs, int nyGlobal, bool a
     if (st == E3D_OK) st = adjoint ? stageSignalsIn(c, r.R, in) : stageSignalsZero(c, r.R);
     if (st == E3D_OK) st = allocFields(c, c->w0, true);
     if (st == E3D_OK) st = allocFields(c, c->w1, true);
+    c->ghosts = true;
     c->tailReady = takesTail(c);
     c->pending = {};
     if (st == E3D_OK && c->tailReady) st = prepareInject(c, c->acqA, adjoint ? r.R.set : r.S.set, false);
@@ -2201,7 +2203,9 @@ static Fields9& ringAt(std::vector<Fields9>& r, long long m) {
   return r[(size_t)(((m % R) + R) % R)];
 }
 
-// Allocate a ring of `levels` levels whose first two are a and b; levels -1 and 0 zeroed.
+// Allocate a ring of `levels` levels whose first two are a and b; levels -1 and 0 zeroed.  The cells
+// around the updated ones read as zero in every level: no step writes them, and a slab run, which
+// does, leaves `ghosts` set.
 static int ensureRing(Context* c, std::vector<Fields9>& ring, Fields9& a, Fields9& b, int levels) {
   if (ring.empty()) {
     E3D_RET(allocFields(c, a, false));
@@ -2215,6 +2219,10 @@ static int ensureRing(Context* c, std::vector<Fields9>& ring, Fields9& a, Fields
     }
   }
   E3D_ARG((int)ring.size() == levels, "ring size changed");
+  if (c->ghosts && &ring == &c->adjRing) {
+    for (auto& f : ring) E3D_RET(zeroFields(c, f));
+    c->ghosts = false;
+  }
   // levels -1 and 0; a step writes every updated cell of the others before it is read
   E3D_RET(zeroFields(c, ring.back()));
   return zeroFields(c, ring.front());

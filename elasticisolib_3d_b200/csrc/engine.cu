@@ -328,7 +328,7 @@ static void hostCopy(char* dst, const char* src, size_t bytes) {
   }
 }
 
-// The source is read when this returns.
+// Pageable sources are read when this returns, pinned and registered ones when the stream is.
 static int copyIn(Context* c, void* dev, const void* host, size_t bytes) {
   if (!staged(c, host, bytes)) {
     E3D_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->st));
@@ -3223,11 +3223,13 @@ int bornForwardHost(Context* c, const float* const* srcSig, float* const* data, 
   E3D_RET(rejectFreeSurface(c));
   E3D_ARG(srcSig && data && pert, "null argument");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
+  for (int k = 0; k < NMED; k++) E3D_ARG(pert[k] != nullptr, "null perturbation plane");
   E3D_RET(ensurePert(c));
-  for (int k = 0; k < NMED; k++)
-    E3D_RET(copyIn(c, c->pertDev[k], pert[k], (size_t)c->cells * sizeof(float)));
   Staged S, R;
-  int st = stageGeom(c, src, false, S);
+  int st = E3D_OK;
+  for (int k = 0; k < NMED && st == E3D_OK; k++)
+    st = copyIn(c, c->pertDev[k], pert[k], (size_t)c->cells * sizeof(float));
+  if (st == E3D_OK) st = stageGeom(c, src, false, S);
   if (st == E3D_OK) st = stageGeom(c, rec, true, R);
   if (st == E3D_OK) st = stageSignalsIn(c, S, srcSig);
   if (st == E3D_OK) st = stageSignalsZero(c, R);
@@ -3238,6 +3240,7 @@ int bornForwardHost(Context* c, const float* const* srcSig, float* const* data, 
     setLastError("stream failure", __FILE__, __LINE__);
     st = E3D_ERR_CUDA;
   }
+  if (st != E3D_OK) cudaStreamSynchronize(c->st);  // copies of the caller's pinned planes end with the call
   releaseStaged(c, S);
   releaseStaged(c, R);
   return st;
@@ -3249,17 +3252,22 @@ int bornAdjointHost(Context* c, const float* const* srcSig, const float* const* 
   E3D_RET(rejectFreeSurface(c));
   E3D_ARG(srcSig && data && pert, "null argument");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
+  for (int k = 0; k < NMED; k++) E3D_ARG(pert[k] != nullptr, "null image plane");
   E3D_RET(ensurePert(c));
   // the reference copies the caller's planes to the device and accumulates
   // the image onto them (BornElasticGpuFunctions_3D.cu:2110-2114)
   const size_t planeBytes = (size_t)c->cells * sizeof(float);
-  for (int k = 0; k < NMED; k++) {
-    E3D_ARG(pert[k] != nullptr, "null image plane");
-    if (fromZero) E3D_CUDA_TRY(cudaMemsetAsync(c->pertDev[k], 0, planeBytes, c->st));
-    else E3D_RET(copyIn(c, c->pertDev[k], pert[k], planeBytes));
-  }
   Staged S, R;
-  int st = stageGeom(c, src, false, S);
+  int st = E3D_OK;
+  for (int k = 0; k < NMED && st == E3D_OK; k++) {
+    if (!fromZero) {
+      st = copyIn(c, c->pertDev[k], pert[k], planeBytes);
+    } else if (cudaMemsetAsync(c->pertDev[k], 0, planeBytes, c->st) != cudaSuccess) {
+      setLastError("clearing the image planes failed", __FILE__, __LINE__);
+      st = E3D_ERR_CUDA;
+    }
+  }
+  if (st == E3D_OK) st = stageGeom(c, src, false, S);
   if (st == E3D_OK) st = stageGeom(c, rec, true, R);
   if (st == E3D_OK) st = stageSignalsIn(c, S, srcSig);
   if (st == E3D_OK) st = stageSignalsIn(c, R, const_cast<float* const*>(data));
@@ -3270,6 +3278,7 @@ int bornAdjointHost(Context* c, const float* const* srcSig, const float* const* 
     if (st == E3D_OK && cudaStreamSynchronize(c->st) != cudaSuccess) st = E3D_ERR_CUDA;
     if (st != E3D_OK) setLastError("copy-out failure", __FILE__, __LINE__);
   }
+  if (st != E3D_OK) cudaStreamSynchronize(c->st);  // copies of the caller's pinned planes end with the call
   releaseStaged(c, S);
   releaseStaged(c, R);
   return st;

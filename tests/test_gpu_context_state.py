@@ -7,8 +7,9 @@ import numpy as np
 import pytest
 
 from cases import random_signals
+from elasticisolib_3d_b200 import _native as N
 from elasticisolib_3d_b200 import synthetic as S
-from elasticisolib_3d_b200.engine import Propagator, SlabPropagator
+from elasticisolib_3d_b200.engine import Propagator, SlabPropagator, _geom
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +60,26 @@ def test_born_image_after_a_slab_run(first):
     _equal(got, fresh.born_adjoint(sig, dat, lspos, lrpos))
     fresh.close()
     sl.close()
+
+
+def test_born_calls_refuse_a_missing_plane():
+    """A null perturbation or image plane is refused with a status, on planes large enough for the
+    staged copies too, and the next call runs."""
+    nz, nx, ny, nts = 168, 168, 152, 3
+    rng = np.random.default_rng(6)
+    pr = _propagator(nz, nx, ny, nts, sub=1)
+    pr.set_medium(_medium(nz, nx, ny))
+    spos = [_points(rng, nz, nx, ny, 4) for _ in range(7)]
+    rpos = [_points(rng, nz, nx, ny, 9) for _ in range(7)]
+    sig, dat = random_signals(spos, nts, rng), random_signals(rpos, nts, rng)
+    pert = [np.ones((ny, nx, nz), np.float32)] * 8
+    SP, SN, k1 = _geom(spos)
+    RP, RN, k2 = _geom(rpos)
+    ref = pr.born_forward(sig, pert, spos, rpos)
+    for hole in (0, 7):
+        planes = [None if k == hole else p for k, p in enumerate(pert)]
+        for name in ("e3d_born_forward", "e3d_born_adjoint"):
+            with pytest.raises(N.E3DError, match="null"):
+                N.call(name, pr.handle, N.ptr_array(sig), N.ptr_array(dat), SP, SN, RP, RN, N.ptr_array(planes))
+    _equal(pr.born_forward(sig, pert, spos, rpos), ref)
+    pr.close()

@@ -107,6 +107,7 @@ struct Context {
   } pending;
   std::unordered_map<unsigned long long, CUtensorMap> tmaps;  // (pointer, box) -> tensor map
   std::vector<void*> owned;  // every device allocation of this context
+  bool allocFailed = false;  // the device had no memory for an allocation of the running pass
   // working wavefields (primary propagation)
   Fields9 w0, w1;
   bool ghosts = false;       // a slab run left its neighbours' planes in the FAT planes of w0 and w1
@@ -164,8 +165,11 @@ static int devAlloc(Context* c, void** p, size_t bytes) {
   if (bytes == 0) bytes = 16;
   cudaError_t e = cudaMallocAsync(p, bytes, c->st);
   if (e != cudaSuccess) {
+    cudaGetLastError();  // not left for the next launch check to find
     setLastError(cudaGetErrorString(e), __FILE__, __LINE__);
-    return e == cudaErrorMemoryAllocation ? E3D_ERR_OOM : E3D_ERR_CUDA;
+    if (e != cudaErrorMemoryAllocation) return E3D_ERR_CUDA;
+    c->allocFailed = true;
+    return E3D_ERR_OOM;
   }
   c->owned.push_back(*p);
   return E3D_OK;
@@ -208,10 +212,8 @@ static void fieldFree(Context* c, float* p) {
   if (p) devFree(c, p - c->fieldOff);
 }
 
-// Gives up the padding of the rows where the device has no memory for it: every field buffer is
-// released (they hold nothing between calls; saved checkpoints become invalid) and the medium moves to
-// unpadded rows, plane by plane.
-static int unpadRows(Context* c) {
+// Releases every field buffer (they hold nothing between calls; saved checkpoints become invalid).
+static int dropFields(Context* c) {
   std::vector<float*> old;
   auto drop = [&](Fields9& f) {
     for (int k = 0; k < NCOMP; k++) {
@@ -242,30 +244,63 @@ static int unpadRows(Context* c) {
   E3D_CUDA_TRY(cudaStreamSynchronize(c->st));
   cudaMemPool_t pool = nullptr;
   if (cudaDeviceGetDefaultMemPool(&pool, c->d.device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
-  const GridConst g = c->g;
-  const int off = c->fieldOff;
-  c->g.pz = (g.nz + 3) / 4 * 4;
-  c->g.yStride = (long long)c->g.pz * g.nx;
-  c->g.n = c->g.yStride * g.ny;
-  c->fieldOff = FAT;
-  for (int k = 0; k < NMED; k++) {
-    if (!c->med[k]) continue;
-    float* m = nullptr;
-    E3D_RET(fieldAlloc(c, &m));
-    E3D_CUDA_TRY(cudaMemcpy2DAsync(m, (size_t)c->g.pz * sizeof(float), c->med[k], (size_t)g.pz * sizeof(float),
-                                   (size_t)g.nz * sizeof(float), (size_t)g.nx * g.ny, cudaMemcpyDeviceToDevice, c->st));
-    devFree(c, c->med[k] - off);
-    c->med[k] = m;
-  }
   return E3D_OK;
 }
 
-// Runs a pass that starts from nothing kept, again without the rows' padding if memory ran out.
+// Rows without padding from here on; the context holds no field and no medium in the old ones.
+static void setUnpadded(Context* c) {
+  GridConst& g = c->g;
+  g.pz = (g.nz + 3) / 4 * 4;
+  g.yStride = (long long)g.pz * g.nx;
+  g.n = g.yStride * g.ny;
+  c->fieldOff = FAT;
+}
+
+// Gives up the padding of the rows where the device has no memory for it: the fields are released and
+// the medium moves to unpadded rows.  All eight planes move or none does: where the device cannot hold
+// both forms of the medium for a moment, it cannot hold the 18 fields of the smallest pass in
+// unpadded rows either, and the context stays as it is.
+static int unpadRows(Context* c) {
+  E3D_RET(dropFields(c));
+  const GridConst g = c->g;
+  const int off = c->fieldOff;
+  float* old[NMED];
+  std::copy(c->med, c->med + NMED, old);
+  setUnpadded(c);
+  int st = E3D_OK;
+  for (int k = 0; k < NMED && st == E3D_OK; k++) {
+    c->med[k] = nullptr;
+    if (!old[k]) continue;
+    st = fieldAlloc(c, &c->med[k]);
+    if (st == E3D_OK && cudaMemcpy2DAsync(c->med[k], (size_t)c->g.pz * sizeof(float), old[k],
+                                          (size_t)g.pz * sizeof(float), (size_t)g.nz * sizeof(float),
+                                          (size_t)g.nx * g.ny, cudaMemcpyDeviceToDevice, c->st) != cudaSuccess) {
+      setLastError("moving the medium failed", __FILE__, __LINE__);
+      st = E3D_ERR_CUDA;
+    }
+  }
+  for (int k = 0; k < NMED; k++) {
+    if (st != E3D_OK) {
+      if (c->med[k] != old[k]) fieldFree(c, c->med[k]);
+      c->med[k] = old[k];
+    } else if (old[k]) {
+      devFree(c, old[k] - off);
+    }
+  }
+  if (st != E3D_OK) {
+    c->g = g;
+    c->fieldOff = off;
+  }
+  return st;
+}
+
+// Runs a pass that starts from nothing kept, again without the rows' padding if the device had no memory
+// for one of its buffers (a plan that does not fit its budget is refused as it is).
 template <class Pass>
 static int withRows(Context* c, Pass pass) {
+  c->allocFailed = false;
   int st = pass();
-  if (st != E3D_ERR_OOM || c->fieldOff == FAT) return st;
-  cudaGetLastError();
+  if (st != E3D_ERR_OOM || !c->allocFailed || c->fieldOff == FAT) return st;
   E3D_RET(unpadRows(c));
   return pass();
 }
@@ -872,7 +907,6 @@ static int prepareInject(Context* c, AcqTable& t, const DevSignals& set, bool pr
   if (set.off[NCOMP] == 0 || set.off[NCOMP] > kTailInjectMax) return E3D_OK;
   const int st = buildAcq(c, t, set, premultiplied, shots);
   if (st != E3D_ERR_OOM) return st;
-  cudaGetLastError();
   t.n = 0;
   return E3D_OK;
 }

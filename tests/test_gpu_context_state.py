@@ -1,10 +1,14 @@
 """GPU: what one call of a context leaves for the next.
 
-A context keeps its buffers between calls.  Passes that follow a slab run give what a fresh context
-gives; they run the same kernels on the same values, so the results are equal bit for bit.
+A context keeps its buffers between calls.  Passes that follow a slab run, a refused call or a failed
+allocation give what a fresh context gives; they run the same kernels on the same values, so the
+results are equal bit for bit.
 """
+import contextlib
+
 import numpy as np
 import pytest
+import torch
 
 from cases import random_signals
 from elasticisolib_3d_b200 import _native as N
@@ -34,6 +38,30 @@ def _propagator(nz, nx, ny, nts, sub=4, pad=3, cls=Propagator, **kw):
 def _equal(a, b):
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x, y)
+
+
+@contextlib.contextmanager
+def _memory_left(nbytes):
+    """All but about `nbytes` of the device's free memory held by another allocation."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - int(nbytes), dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        torch.cuda.synchronize()
+        del hog
+        torch.cuda.empty_cache()
+
+
+def _device_sets(rng, nz, nx, ny, nts, nsrc=5, nrec=200):
+    """Explosive sources and pressure-like receivers as device tables, and random source signals."""
+    s = _points(rng, nz, nx, ny, nsrc)
+    r = np.unique(np.concatenate([s, _points(rng, nz, nx, ny, nrec)]))
+    so = [len(s) * min(max(k - 3, 0), 3) for k in range(10)]
+    ro = [len(r) * min(max(k - 3, 0), 3) for k in range(10)]
+    sig = torch.from_numpy(rng.standard_normal((nts, so[9])).astype(np.float32)).cuda()
+    return torch.from_numpy(np.tile(s, 3)).cuda(), so, torch.from_numpy(np.tile(r, 3)).cuda(), ro, sig
 
 
 @pytest.mark.parametrize("first", [False, True])
@@ -82,4 +110,52 @@ def test_born_calls_refuse_a_missing_plane():
             with pytest.raises(N.E3DError, match="null"):
                 N.call(name, pr.handle, N.ptr_array(sig), N.ptr_array(dat), SP, SN, RP, RN, N.ptr_array(planes))
     _equal(pr.born_forward(sig, pert, spos, rpos), ref)
+    pr.close()
+
+
+def test_failed_allocation_leaves_the_medium():
+    """A call that runs out of memory, whatever it gave up on the way, leaves a medium that the next
+    call propagates in."""
+    nz, nx, ny, nts = 72, 400, 800, 4
+    rng = np.random.default_rng(2)
+    med = _medium(nz, nx, ny)
+    sp, so, rp, ro, sig = _device_sets(rng, nz, nx, ny, nts)
+    out = []
+    for short in (False, True):
+        pr = _propagator(nz, nx, ny, nts)
+        pr.set_medium(med)
+        rec = torch.empty((nts, ro[9]), device="cuda")
+        with pytest.raises(N.E3DError):  # refused; the position check has its word of memory from here on
+            pr.nl_propagate_device(False, torch.zeros_like(sp), so, rp, ro, sig, rec)
+        pr.synchronize()
+        if short:
+            with _memory_left(8 << 20):
+                with pytest.raises(N.E3DError):
+                    pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
+        pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
+        pr.synchronize()
+        out.append(rec.cpu().numpy())
+        pr.close()
+    assert np.abs(out[0]).max() > 0
+    np.testing.assert_array_equal(out[1], out[0])
+
+
+def test_refused_plan_keeps_the_buffers():
+    """A budget that no plan fits is refused without giving up what the context holds: a propagation
+    before and after it uses the same memory."""
+    nz, nx, ny, nts = 72, 200, 400, 4
+    rng = np.random.default_rng(7)
+    pr = _propagator(nz, nx, ny, nts)
+    pr.set_medium(_medium(nz, nx, ny))
+    sp, so, rp, ro, sig = _device_sets(rng, nz, nx, ny, nts)
+    rec = torch.empty((nts, ro[9]), device="cuda")
+    pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
+    pr.set_checkpoint_policy("auto", 0, 1.0)
+    with pytest.raises(N.E3DError):
+        pr.fwi_forward_device(sp, so, rp, ro, sig, rec)
+    pr.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
+    pr.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 4 * nz * nx * ny
     pr.close()

@@ -2525,31 +2525,42 @@ static int bornForwardDevice(Context* c, const DevSignals& srcSet, const DevSign
 // goes, so the adjoint pass recomputes every segment but the last (which is
 // the longest, hence the end alignment).
 // The plan (segment length, checkpoint storage, velocity-slot storage) is
-// schedule::choosePlan's for the memory budget autoBudget gives.
+// schedule::choosePlan's for the memory budget autoBudget gives, on the grid's own
+// cells: the padding of the rows takes no part in it.  16-bit copies are kept
+// without the padding; where the padding of the others has no room beside the
+// plan, the padding goes and the plan stays.
 // ---------------------------------------------------------------------------
 enum { V_F32 = 0, V_F16 = 1 };
 
 using schedule::segStart;
 
-static size_t ckptBytesPerState(const Context* c, int type) {
-  return (size_t)schedule::stateBytes(c->g.n, c->d.ny, type);
-}
-static size_t vHalfBytes(const Context* c) { return schedule::halfSlotValuesBytes(c->g.n); }
-static size_t vStoreBytes(const Context* c) { return schedule::halfSlotBytes(c->g.n, c->d.ny); }
-static double vSlotBytes(const Context* c, int vt) { return schedule::slotBytes(c->g.n, c->d.ny, vt); }
+// Cells of a field in unpadded rows (of 16 bytes), as 16-bit copies hold them.
+static long long packedCells(const Context* c) { return (long long)((c->d.nz + 3) / 4 * 4) * c->d.nx * c->d.ny; }
 
-static double heldBytes(const Context* c) {
+static size_t ckptBytesPerState(const Context* c, int type) {
+  return (size_t)schedule::stateBytes(type == CKPT_F32 ? c->g.n : packedCells(c), c->d.ny, type);
+}
+static size_t vHalfBytes(const Context* c) { return schedule::halfSlotValuesBytes(packedCells(c)); }
+static size_t vStoreBytes(const Context* c) { return schedule::halfSlotBytes(packedCells(c), c->d.ny); }
+static double vSlotBytes(const Context* c, int vt) {
+  return vt == V_F32 ? schedule::slotBytes(c->g.n, c->d.ny, vt) : (double)vStoreBytes(c);
+}
+
+// Bytes of the checkpoints and velocity slots this context holds, as they are or without padding.
+static double heldBytes(const Context* c, bool padded) {
+  const int type = c->ckptAllocType, ny = c->d.ny;
   double b = 0;
   for (void* p : c->ckpt)
-    if (p) b += ckptBytesPerState(c, c->ckptAllocType);
-  b += (double)c->vSlots.size() * vSlotBytes(c, V_F32) + (double)c->vStore.size() * vSlotBytes(c, V_F16);
+    if (p) b += padded ? ckptBytesPerState(c, type) : schedule::stateBytes(c->cells, ny, type);
+  b += (double)c->vSlots.size() * (padded ? vSlotBytes(c, V_F32) : schedule::slotBytes(c->cells, ny, V_F32));
+  b += (double)c->vStore.size() * (padded ? vSlotBytes(c, V_F16) : schedule::slotBytes(c->cells, ny, V_F16));
   return b;
 }
 
 // Device bytes the adjoint pass will still allocate (adjoint levels, decimation
-// slots, premultiplied levels).
-static double pendingAdjointBytes(const Context* c) {
-  const double f = (double)c->g.n * sizeof(float);
+// slots, premultiplied levels), fields of n cells.
+static double pendingAdjointBytes(const Context* c, long long n) {
+  const double f = (double)n * sizeof(float);
   double b = 0;
   const int R = ringLevels(c);
   if (R) {
@@ -2565,29 +2576,49 @@ static double pendingAdjointBytes(const Context* c) {
   return b;
 }
 
-// Bytes available for checkpoints and velocity slots: the explicit budget, or
-// 85% of the free memory left after the caller's reserve (negative budget)
-// and the adjoint pass's pending allocations.
-static double autoBudget(const Context* c, size_t free) {
+// What the padding of everything held adds to its bytes.
+static double paddingHeld(const Context* c) {
+  int levels = 0;
+  auto held = [&](const Fields9& f) { levels += f.p[0] ? 1 : 0; };
+  if (c->srcRing.empty()) held(c->s0), held(c->s1);
+  if (c->adjRing.empty()) held(c->w0), held(c->w1);
+  for (auto* ring : {&c->srcRing, &c->adjRing})
+    for (const Fields9& f : *ring) held(f);
+  for (const Fields9* f : {&c->ss[0], &c->ss[1], &c->q0, &c->q1}) held(*f);
+  const double fields = (double)NCOMP * (levels + 2 * c->batchShots) + NMED;
+  return fields * (double)(c->g.n - c->cells) * sizeof(float) + heldBytes(c, true) - heldBytes(c, false);
+}
+
+// Bytes available for checkpoints and velocity slots: the explicit budget, or a share (85%) of the free
+// memory left after the caller's reserve (negative budget), less the adjoint pass's pending allocations
+// in fields of n cells.
+static double autoBudget(const Context* c, double free, double share, long long n) {
   if (c->budget > 0) return c->budget;
   const double reserve = c->budget < 0 ? -c->budget : 0.0;
-  return 0.85 * ((double)free - reserve) - pendingAdjointBytes(c);
+  return share * (free - reserve) - pendingAdjointBytes(c, n);
 }
 
 static int choosePlan(Context* c, int& L) {
   size_t free = 0, total = 0;
   E3D_CUDA_TRY(cudaMemGetInfo(&free, &total));
   // memory this context already holds for checkpoints and velocity slots counts as available
-  const double budget = autoBudget(c, free) + heldBytes(c);
+  const double budget = autoBudget(c, (double)free + paddingHeld(c), 0.85, c->cells) + heldBytes(c, false);
   schedule::Plan plan{};
-  if (!schedule::choosePlan(c->g.n, c->d.ny, c->d.nts, budget, c->ckptType, c->vType, c->segment, plan)) {
+  if (!schedule::choosePlan(c->cells, c->d.ny, c->d.nts, budget, c->ckptType, c->vType, c->segment, plan)) {
     setLastError("wavefield checkpoints do not fit in device memory", __FILE__, __LINE__);
     return E3D_ERR_OOM;
   }
   c->ckptUsed = plan.ck;
   c->vUsed = plan.vt;
   L = plan.L;
-  return E3D_OK;
+  if (c->fieldOff == FAT) return E3D_OK;
+  // the plan in padded rows: within an explicit budget, or (automatic) within 95% of the memory
+  const int nseg = schedule::segments(c->d.nts - 1, L);
+  const bool half = plan.vt == V_F16;
+  const double need = (double)(nseg - 1) * ckptBytesPerState(c, plan.ck) + (half ? 4 : L + 3) * vSlotBytes(c, V_F32) +
+                      (half ? (L + 2) * vSlotBytes(c, V_F16) : 0.0);
+  if (need <= autoBudget(c, (double)free, 0.95, c->g.n) + heldBytes(c, true)) return E3D_OK;
+  return unpadRows(c);
 }
 
 static int resizeVStorage(Context* c, int nF32, int nF16) {
@@ -2608,45 +2639,46 @@ static int resizeVStorage(Context* c, int nF32, int nF16) {
   return E3D_OK;
 }
 
+static SliceRows sliceRows(const Context* c) {
+  SliceRows s;
+  s.rv = (unsigned)(c->d.nz + 3) / 4;
+  s.fv = (unsigned)c->g.pz / 4;
+  s.rows = (unsigned)c->d.nx;
+  s.n = c->g.n;
+  s.ys = c->g.yStride;
+  s.pn = packedCells(c);
+  s.pys = s.pn / c->d.ny;
+  return s;
+}
+
 // Grid of the slice kernels for nf consecutive fields: each block covers
-// kSliceThreads * kSliceVecPerThread * 4 values of one y slice.
-static dim3 sliceGrid(const Context* c, int nf) {
-  const long long per = (long long)kSliceThreads * kSliceVecPerThread * 4;
-  return dim3((unsigned)((c->g.yStride + per - 1) / per), (unsigned)c->d.ny, (unsigned)nf);
+// kSliceThreads * kSliceVecPerThread vectors of one y slice.
+static dim3 sliceGrid(const SliceRows& s, const Context* c, int nf) {
+  const unsigned per = kSliceThreads * kSliceVecPerThread;
+  return dim3((s.rv * s.rows + per - 1) / per, (unsigned)c->d.ny, (unsigned)nf);
 }
 
-// Four-wide slice access: slices and fields start on 4-value boundaries and
-// the FP32 and 16-bit arrays are 16- and 8-byte aligned.
-static bool sliceVec(const Context* c, const void* f32, const void* h16) {
-  return c->g.yStride % 4 == 0 && c->g.n % 4 == 0 && (uintptr_t)f32 % 16 == 0 && (uintptr_t)h16 % 8 == 0;
-}
-
-// Scaled 16-bit copy of nf consecutive fields of n values: slice maxima into
-// the scratch, then the packed values and one unscaling factor per (field, y).
+// Scaled 16-bit copy of nf consecutive fields: slice maxima into the scratch,
+// then the packed values and one unscaling factor per (field, y).
 template <typename H>
 static int packSlices(Context* c, const float* a, int nf, int topExp, H* out, float* scales) {
-  const long long n = c->g.n, ys = c->g.yStride;
+  const SliceRows s = sliceRows(c);
   float* smax = (float*)c->scratch;
-  const dim3 grid = sliceGrid(c, nf);
-  const bool vec = sliceVec(c, a, out);
+  const dim3 grid = sliceGrid(s, c, nf);
   E3D_CUDA_TRY(cudaMemsetAsync(smax, 0, (size_t)nf * c->d.ny * sizeof(float), c->st));
   c->launches += 2;
-  if (vec) kSliceMaxAbs<true><<<grid, kSliceThreads, 0, c->st>>>(a, n, ys, smax);
-  else kSliceMaxAbs<false><<<grid, kSliceThreads, 0, c->st>>>(a, n, ys, smax);
+  kSliceMaxAbs<<<grid, kSliceThreads, 0, c->st>>>(a, s, smax);
   E3D_LAUNCH_CHECK();
-  if (vec) kPackSlices<H, true><<<grid, kSliceThreads, 0, c->st>>>(a, n, ys, smax, topExp, out, scales);
-  else kPackSlices<H, false><<<grid, kSliceThreads, 0, c->st>>>(a, n, ys, smax, topExp, out, scales);
+  kPackSlices<H><<<grid, kSliceThreads, 0, c->st>>>(a, s, smax, topExp, out, scales);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
 
 template <typename H>
 static int unpackSlices(Context* c, const H* in, int nf, const float* scales, float* a) {
-  const long long n = c->g.n, ys = c->g.yStride;
-  const dim3 grid = sliceGrid(c, nf);
+  const SliceRows s = sliceRows(c);
   c->launches++;
-  if (sliceVec(c, a, in)) kUnpackSlices<H, true><<<grid, kSliceThreads, 0, c->st>>>(in, n, ys, scales, a);
-  else kUnpackSlices<H, false><<<grid, kSliceThreads, 0, c->st>>>(in, n, ys, scales, a);
+  kUnpackSlices<H><<<sliceGrid(s, c, nf), kSliceThreads, 0, c->st>>>(in, s, scales, a);
   E3D_LAUNCH_CHECK();
   return E3D_OK;
 }
@@ -2663,7 +2695,7 @@ static int unpackVelocity(Context* c, const void* store, float* v) {
 }
 
 static int packState(Context* c, int seg) {
-  const long long n = c->g.n;
+  const long long n = c->g.n, pn = packedCells(c);
   const int ny = c->d.ny;
   Fields9* parts[2] = {&c->s0, &c->s1};
   if (c->ckptUsed == CKPT_F32) {
@@ -2679,16 +2711,16 @@ static int packState(Context* c, int seg) {
     for (int k = 0; k < NCOMP; k++) {
       const int f = h * NCOMP + k;
       if (c->ckptUsed == CKPT_F16)
-        E3D_RET(packSlices(c, parts[h]->p[k], 1, 14, (__half*)c->ckpt[seg] + (size_t)f * n, scales + (size_t)f * ny));
+        E3D_RET(packSlices(c, parts[h]->p[k], 1, 14, (__half*)c->ckpt[seg] + (size_t)f * pn, scales + (size_t)f * ny));
       else
-        E3D_RET(packSlices(c, parts[h]->p[k], 1, 0, (__nv_bfloat16*)c->ckpt[seg] + (size_t)f * n,
+        E3D_RET(packSlices(c, parts[h]->p[k], 1, 0, (__nv_bfloat16*)c->ckpt[seg] + (size_t)f * pn,
                            scales + (size_t)f * ny));
     }
   return E3D_OK;
 }
 
 static int unpackState(Context* c, int seg) {
-  const long long n = c->g.n;
+  const long long n = c->g.n, pn = packedCells(c);
   const int ny = c->d.ny;
   Fields9* parts[2] = {&c->s0, &c->s1};
   for (int h = 0; h < 2; h++)
@@ -2698,18 +2730,18 @@ static int unpackState(Context* c, int seg) {
         E3D_CUDA_TRY(cudaMemcpyAsync(parts[h]->p[k], (float*)c->ckpt[seg] + (size_t)f * n, n * sizeof(float),
                                      cudaMemcpyDeviceToDevice, c->st));
       else if (c->ckptUsed == CKPT_F16)
-        E3D_RET(unpackSlices(c, (const __half*)c->ckpt[seg] + (size_t)f * n, 1, c->ckptScale[seg] + (size_t)f * ny,
+        E3D_RET(unpackSlices(c, (const __half*)c->ckpt[seg] + (size_t)f * pn, 1, c->ckptScale[seg] + (size_t)f * ny,
                              parts[h]->p[k]));
       else
-        E3D_RET(unpackSlices(c, (const __nv_bfloat16*)c->ckpt[seg] + (size_t)f * n, 1,
+        E3D_RET(unpackSlices(c, (const __nv_bfloat16*)c->ckpt[seg] + (size_t)f * pn, 1,
                              c->ckptScale[seg] + (size_t)f * ny, parts[h]->p[k]));
     }
   return E3D_OK;
 }
 
-static int prepareCheckpoints(Context* c, int& L, int& nseg) {
+// Buffers of the plan that choosePlan made.
+static int prepareCheckpoints(Context* c, int L, int& nseg) {
   const int blocks = c->d.nts - 1;
-  E3D_RET(choosePlan(c, L));
   nseg = (blocks + L - 1) / L;
   if (c->ckptSegLen != L || (int)c->ckpt.size() != nseg || c->ckptAllocType != c->ckptUsed ||
       c->vAllocType != c->vUsed) {
@@ -2721,8 +2753,8 @@ static int prepareCheckpoints(Context* c, int& L, int& nseg) {
     E3D_RET(resizeVStorage(c, c->vUsed == V_F32 ? L + 3 : 4, c->vUsed == V_F32 ? 0 : L + 2));
     c->vAllocType = c->vUsed;
     for (int s = 1; s < nseg; s++) {
-      const size_t eb = c->ckptUsed == CKPT_F32 ? 4 : 2;
-      E3D_RET(devAlloc(c, &c->ckpt[s], (size_t)18 * c->g.n * eb));
+      const size_t bytes = c->ckptUsed == CKPT_F32 ? (size_t)4 * c->g.n : (size_t)2 * packedCells(c);
+      E3D_RET(devAlloc(c, &c->ckpt[s], 18 * bytes));
       if (c->ckptUsed != CKPT_F32)
         E3D_RET(devAlloc(c, (void**)&c->ckptScale[s], (size_t)18 * c->d.ny * sizeof(float)));
     }
@@ -2776,6 +2808,7 @@ static int sourcePassWithCheckpoints(Context* c, const DevSignals& srcSet, const
   int L = 0, nseg = 0;
   c->ckptValid = false;
   c->tailValid = false;
+  E3D_RET(choosePlan(c, L));
   E3D_RET(prepareCheckpoints(c, L, nseg));
   E3D_RET(allocFields(c, c->s0, true));
   E3D_RET(allocFields(c, c->s1, true));
@@ -3016,6 +3049,8 @@ static int sourcePassRing(Context* c, const DevSignals& srcSet, const DevSignals
     bool prem = false;  // known before the plan, which then leaves out the dual state's levels
     E3D_RET(premultipliedAdjoint(c, prem));
   }
+  E3D_RET(choosePlan(c, L));
+  E3D_RET(ensureRing(c, c->srcRing, c->s0, c->s1, ringLevels(c)));  // anew if the rows changed
   c->tailReady = takesTail(c);
   c->pending = {};
   if (c->tailReady) E3D_RET(prepareInject(c, c->acqA, srcSet, false));

@@ -2597,14 +2597,46 @@ __global__ void __launch_bounds__(TZ * ITX, ITX == 4 ? 3 : 1) kImagingLev(const 
 // bf16 with one fp32 scale per (field, y) slice (max-abs / 2^14 for fp16,
 // max-abs for bf16), or copied raw in fp32.
 // ---------------------------------------------------------------------------
-// Slice maxima, packing and unpacking run on a (chunk, y slice, field) grid:
-// nf fields of n values each, slice y of field f at f*n + y*ys.  With VEC the
-// slices are read and written four values at a time (ys and n multiples of 4,
-// 16-byte aligned fields).
+// Slice maxima, packing and unpacking run on a (chunk, y slice, field) grid over nf fields.  The
+// 16-bit copy is kept in rows of rv four-cell vectors without the fields' padding, which streams gain
+// nothing from and which a memory plan would pay for.
+struct SliceRows {
+  unsigned rv;         // vectors per packed row, (nz + 3) / 4
+  unsigned fv;         // vectors per field row (its pitch)
+  unsigned rows;       // nx
+  long long n, ys;     // cells per field and per y slice of the fields
+  long long pn, pys;   // the same of the packed copy
+};
 constexpr int kSliceThreads = 256;
 constexpr int kSliceVecPerThread = 4;
 
-__device__ __forceinline__ unsigned sliceChunkBegin() { return blockIdx.x * kSliceThreads + threadIdx.x; }
+// Vectors of one slice that a thread visits: packed index j, field index i (one division per thread,
+// the steps are added).
+struct SliceCursor {
+  unsigned j, i, z, end, stride, di, dz, rv, gap;
+  __device__ __forceinline__ explicit SliceCursor(const SliceRows& s) {
+    rv = s.rv;
+    gap = s.fv - s.rv;
+    end = s.rows * s.rv;
+    stride = gridDim.x * kSliceThreads;
+    j = blockIdx.x * kSliceThreads + threadIdx.x;
+    const unsigned r = j / rv, dr = stride / rv;
+    z = j - r * rv;
+    i = j + r * gap;
+    dz = stride - dr * rv;
+    di = stride + dr * gap;
+  }
+  __device__ __forceinline__ bool in() const { return j < end; }
+  __device__ __forceinline__ void next() {
+    j += stride;
+    i += di;
+    z += dz;
+    if (z >= rv) {
+      z -= rv;
+      i += gap;
+    }
+  }
+};
 
 // 16-bit storage types as raw bits, so that four values move as one 8-byte word
 __device__ __forceinline__ unsigned halfBits(__half h) { return __half_as_ushort(h); }
@@ -2623,20 +2655,12 @@ __device__ __forceinline__ float halfValue<__nv_bfloat16>(unsigned bits) {
 // out[f*ny + y] = max |a| over slice y of field f; out must be zeroed first.
 // NaN values are ignored, as by fmaxf; the block maxima combine through an
 // unsigned atomicMax, which orders non-negative floats by their bit patterns.
-template <bool VEC>
-__global__ void __launch_bounds__(kSliceThreads) kSliceMaxAbs(const float* a, long long n, long long ys, float* out) {
-  const long long base = (long long)blockIdx.z * n + (long long)blockIdx.y * ys;
-  const unsigned stride = gridDim.x * kSliceThreads;
+__global__ void __launch_bounds__(kSliceThreads) kSliceMaxAbs(const float* a, SliceRows s, float* out) {
+  const float4* v = reinterpret_cast<const float4*>(a + (long long)blockIdx.z * s.n + (long long)blockIdx.y * s.ys);
   float m = 0.0f;
-  if (VEC) {
-    const float4* v = reinterpret_cast<const float4*>(a + base);
-    const unsigned nv = (unsigned)(ys / 4);
-    for (unsigned j = sliceChunkBegin(); j < nv; j += stride) {
-      const float4 q = __ldg(v + j);
-      m = fmaxf(fmaxf(m, fabsf(q.x)), fmaxf(fabsf(q.y), fmaxf(fabsf(q.z), fabsf(q.w))));
-    }
-  } else {
-    for (long long j = sliceChunkBegin(); j < ys; j += stride) m = fmaxf(m, fabsf(__ldg(a + base + j)));
+  for (SliceCursor c(s); c.in(); c.next()) {
+    const float4 q = __ldg(v + c.i);
+    m = fmaxf(fmaxf(m, fabsf(q.x)), fmaxf(fabsf(q.y), fmaxf(fabsf(q.z), fabsf(q.w))));
   }
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   __shared__ float red[kSliceThreads / 32];
@@ -2655,11 +2679,10 @@ __global__ void __launch_bounds__(kSliceThreads) kSliceMaxAbs(const float* a, lo
 // clamped to +-126 so that slices whose maximum is tiny or subnormal (far from
 // the wavefront) keep finite scales.  A zero or non-finite maximum stores zeros.
 // scales[f*ny + y] receives the unscaling factor.
-template <typename H, bool VEC>
-__global__ void __launch_bounds__(kSliceThreads) kPackSlices(const float* a, long long n, long long ys,
-                                                             const float* smax, int topExp, H* out, float* scales) {
+template <typename H>
+__global__ void __launch_bounds__(kSliceThreads) kPackSlices(const float* a, SliceRows g, const float* smax,
+                                                             int topExp, H* out, float* scales) {
   const size_t slice = (size_t)blockIdx.z * gridDim.y + blockIdx.y;
-  const long long base = (long long)blockIdx.z * n + (long long)blockIdx.y * ys;
   const float m = smax[slice];
   float s = 0.0f, inv = 0.0f;
   if (m > 0.0f && isfinite(m)) {
@@ -2670,38 +2693,25 @@ __global__ void __launch_bounds__(kSliceThreads) kPackSlices(const float* a, lon
     inv = ldexpf(1.0f, -sh);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) scales[slice] = inv;
-  const unsigned stride = gridDim.x * kSliceThreads;
-  if (VEC) {
-    const float4* v = reinterpret_cast<const float4*>(a + base);
-    const unsigned nv = (unsigned)(ys / 4);
-    for (unsigned j = sliceChunkBegin(); j < nv; j += stride) {
-      const float4 q = __ldg(v + j);
-      const uint2 w = make_uint2(halfBits(H(q.x * s)) | halfBits(H(q.y * s)) << 16,
-                                 halfBits(H(q.z * s)) | halfBits(H(q.w * s)) << 16);
-      *reinterpret_cast<uint2*>(out + base + 4 * (long long)j) = w;
-    }
-  } else {
-    for (long long j = sliceChunkBegin(); j < ys; j += stride) out[base + j] = H(__ldg(a + base + j) * s);
+  const float4* v = reinterpret_cast<const float4*>(a + (long long)blockIdx.z * g.n + (long long)blockIdx.y * g.ys);
+  uint2* o = reinterpret_cast<uint2*>(out + (long long)blockIdx.z * g.pn + (long long)blockIdx.y * g.pys);
+  for (SliceCursor c(g); c.in(); c.next()) {
+    const float4 q = __ldg(v + c.i);
+    o[c.j] = make_uint2(halfBits(H(q.x * s)) | halfBits(H(q.y * s)) << 16,
+                        halfBits(H(q.z * s)) | halfBits(H(q.w * s)) << 16);
   }
 }
 
-template <typename H, bool VEC>
-__global__ void __launch_bounds__(kSliceThreads) kUnpackSlices(const H* in, long long n, long long ys,
-                                                               const float* scales, float* a) {
-  const size_t slice = (size_t)blockIdx.z * gridDim.y + blockIdx.y;
-  const long long base = (long long)blockIdx.z * n + (long long)blockIdx.y * ys;
-  const float sc = scales[slice];
-  const unsigned stride = gridDim.x * kSliceThreads;
-  if (VEC) {
-    float4* v = reinterpret_cast<float4*>(a + base);
-    const unsigned nv = (unsigned)(ys / 4);
-    for (unsigned j = sliceChunkBegin(); j < nv; j += stride) {
-      const uint2 w = __ldg(reinterpret_cast<const uint2*>(in + base + 4 * (long long)j));
-      v[j] = make_float4(halfValue<H>(w.x & 0xffffu) * sc, halfValue<H>(w.x >> 16) * sc,
+template <typename H>
+__global__ void __launch_bounds__(kSliceThreads) kUnpackSlices(const H* in, SliceRows g, const float* scales,
+                                                               float* a) {
+  const float sc = scales[(size_t)blockIdx.z * gridDim.y + blockIdx.y];
+  const uint2* v = reinterpret_cast<const uint2*>(in + (long long)blockIdx.z * g.pn + (long long)blockIdx.y * g.pys);
+  float4* o = reinterpret_cast<float4*>(a + (long long)blockIdx.z * g.n + (long long)blockIdx.y * g.ys);
+  for (SliceCursor c(g); c.in(); c.next()) {
+    const uint2 w = __ldg(v + c.j);
+    o[c.i] = make_float4(halfValue<H>(w.x & 0xffffu) * sc, halfValue<H>(w.x >> 16) * sc,
                          halfValue<H>(w.y & 0xffffu) * sc, halfValue<H>(w.y >> 16) * sc);
-    }
-  } else {
-    for (long long j = sliceChunkBegin(); j < ys; j += stride) a[base + j] = float(in[base + j]) * sc;
   }
 }
 

@@ -13,7 +13,7 @@ import torch
 from cases import random_signals
 from elasticisolib_3d_b200 import _native as N
 from elasticisolib_3d_b200 import synthetic as S
-from elasticisolib_3d_b200.engine import Propagator, SlabPropagator, _geom
+from elasticisolib_3d_b200.engine import Propagator, SlabPropagator, _geom, checkpoint_plan
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -158,4 +158,22 @@ def test_refused_plan_keeps_the_buffers():
     pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
     pr.synchronize()
     assert before - torch.cuda.mem_get_info()[0] < 4 * nz * nx * ny
+    pr.close()
+
+
+@pytest.mark.parametrize("nz,nx,ny,nts,budget", [(104, 104, 96, 300, 4.0e9), (72, 100, 100, 400, 3.6e9),
+                                                 (65, 70, 80, 200, 0.95e9), (104, 104, 96, 300, 2.0e9),
+                                                 (104, 104, 96, 300, 1.0e9)])
+def test_rows_do_not_change_the_memory_plan(nz, nx, ny, nts, budget):
+    """The plan of the checkpointed passes is the one of the grid's own cells (checkpoint_plan),
+    however the context lays out its rows."""
+    rng = np.random.default_rng(4)
+    pr = _propagator(nz, nx, ny, nts)
+    pr.set_medium(_medium(nz, nx, ny))
+    pr.set_checkpoint_policy("auto", 0, budget)
+    sp, so, rp, ro, sig = _device_sets(rng, nz, nx, ny, nts)
+    pr.fwi_forward_device(sp, so, rp, ro, sig, torch.empty((nts, ro[9]), device="cuda"))
+    pr.synchronize()
+    want = checkpoint_plan(nz * nx * ny, ny, nts, budget)
+    assert (pr.checkpoint_type, pr.velocity_storage, pr.checkpoint_segment) == want[:3]
     pr.close()

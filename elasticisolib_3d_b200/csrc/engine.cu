@@ -149,6 +149,7 @@ struct Context {
   // pinned staging of large copies between the device and callers' pageable memory (HostCopy)
   char* stage[2] = {};
   cudaEvent_t stageEv[2] = {};
+  size_t stageBytes = 0, stageMoved = 0;  // size of each buffer; bytes copied through them
   // scratch for transposes / signal staging
   void* scratch = nullptr;
   size_t scratchBytes = 0;
@@ -330,26 +331,48 @@ static int zeroFields(Context* c, Fields9& f, int ncomp = NCOMP) {
 // alternate between the bus and a memcpy over several host threads.  Small copies and callers' pinned
 // memory go straight to cudaMemcpyAsync.
 // ---------------------------------------------------------------------------
-constexpr size_t kStageBytes = (size_t)8 << 20;
+//
+// Pinning costs about a millisecond for two buffers of 1 MB and 8 to 12 for two of 8 MB, which move 17 MB
+// in 0.49 ms where the small ones take 0.64, and more so out to untouched pages, which the host threads
+// fault in side by side only across several MB (a Born adjoint call that fetches eight planes of 17 MB:
+// 38.4 against 51.5 ms).  A context starts with the small ones and takes the large ones once the copies it
+// has made would have paid for them: kStageEarned bytes, those out counted four times.
+constexpr size_t kStageSmall = (size_t)1 << 20, kStageLarge = (size_t)8 << 20, kStageEarned = (size_t)1 << 29;
 
-static bool staged(Context* c, const void* host, size_t bytes) {
-  // the buffers cost about 10 ms to pin: only a copy that earns them back makes them
-  if (bytes < (c->stage[1] ? kStageBytes / 2 : 2 * kStageBytes)) return false;
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
-  else if (at.type != cudaMemoryTypeUnregistered) return false;
+static bool stageBuffers(Context* c, size_t bytes) {
+  char* p[2] = {};
   for (int i = 0; i < 2; i++) {
-    if (!c->stage[i] && cudaHostAlloc((void**)&c->stage[i], kStageBytes, cudaHostAllocDefault) != cudaSuccess) {
-      c->stage[i] = nullptr;
-      cudaGetLastError();
-      return false;
-    }
     if (!c->stageEv[i] && cudaEventCreateWithFlags(&c->stageEv[i], cudaEventDisableTiming) != cudaSuccess) {
       c->stageEv[i] = nullptr;
       cudaGetLastError();
       return false;
     }
+    if (cudaHostAlloc((void**)&p[i], bytes, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      if (i) cudaFreeHost(p[0]);
+      return false;
+    }
   }
+  for (int i = 0; i < 2; i++) {
+    if (c->stage[i]) {
+      cudaEventSynchronize(c->stageEv[i]);  // the buffer's last copy
+      cudaFreeHost(c->stage[i]);
+    }
+    c->stage[i] = p[i];
+  }
+  c->stageBytes = bytes;
+  return true;
+}
+
+static bool staged(Context* c, const void* host, size_t bytes, bool out) {
+  if (bytes < (c->stageBytes ? kStageLarge / 2 : 2 * kStageLarge)) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
+  else if (at.type != cudaMemoryTypeUnregistered) return false;
+  if (!c->stageBytes && !stageBuffers(c, kStageSmall)) return false;
+  // without memory for the large buffers the small ones go on
+  if (c->stageBytes < kStageLarge && c->stageMoved >= kStageEarned && !stageBuffers(c, kStageLarge)) c->stageMoved = 0;
+  c->stageMoved += out ? 4 * bytes : bytes;
   return true;
 }
 
@@ -365,13 +388,14 @@ static void hostCopy(char* dst, const char* src, size_t bytes) {
 
 // Pageable sources are read when this returns, pinned and registered ones when the stream is.
 static int copyIn(Context* c, void* dev, const void* host, size_t bytes) {
-  if (!staged(c, host, bytes)) {
+  if (!staged(c, host, bytes, false)) {
     E3D_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->st));
     return E3D_OK;
   }
+  const size_t part = c->stageBytes;
   int i = 0;
-  for (size_t o = 0; o < bytes; o += kStageBytes, i ^= 1) {
-    const size_t n = std::min(kStageBytes, bytes - o);
+  for (size_t o = 0; o < bytes; o += part, i ^= 1) {
+    const size_t n = std::min(part, bytes - o);
     E3D_CUDA_TRY(cudaEventSynchronize(c->stageEv[i]));  // the buffer's last copy
     hostCopy(c->stage[i], (const char*)host + o, n);
     E3D_CUDA_TRY(cudaMemcpyAsync((char*)dev + o, c->stage[i], n, cudaMemcpyHostToDevice, c->st));
@@ -382,14 +406,14 @@ static int copyIn(Context* c, void* dev, const void* host, size_t bytes) {
 
 // Staged copies are complete when this returns, the others when the stream is.
 static int copyOut(Context* c, void* host, const void* dev, size_t bytes) {
-  if (!staged(c, host, bytes)) {
+  if (!staged(c, host, bytes, true)) {
     E3D_CUDA_TRY(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->st));
     return E3D_OK;
   }
-  const size_t chunks = (bytes + kStageBytes - 1) / kStageBytes;
+  const size_t part = c->stageBytes, chunks = (bytes + part - 1) / part;
   auto fetch = [&](size_t k) -> int {
-    const size_t o = k * kStageBytes;
-    E3D_CUDA_TRY(cudaMemcpyAsync(c->stage[k % 2], (const char*)dev + o, std::min(kStageBytes, bytes - o),
+    const size_t o = k * part;
+    E3D_CUDA_TRY(cudaMemcpyAsync(c->stage[k % 2], (const char*)dev + o, std::min(part, bytes - o),
                                  cudaMemcpyDeviceToHost, c->st));
     E3D_CUDA_TRY(cudaEventRecord(c->stageEv[k % 2], c->st));
     return E3D_OK;
@@ -397,9 +421,9 @@ static int copyOut(Context* c, void* host, const void* dev, size_t bytes) {
   for (int i = 0; i < 2; i++) E3D_CUDA_TRY(cudaEventSynchronize(c->stageEv[i]));
   for (size_t k = 0; k < std::min<size_t>(chunks, 2); k++) E3D_RET(fetch(k));
   for (size_t k = 0; k < chunks; k++) {
-    const size_t o = k * kStageBytes;
+    const size_t o = k * part;
     E3D_CUDA_TRY(cudaEventSynchronize(c->stageEv[k % 2]));
-    hostCopy((char*)host + o, c->stage[k % 2], std::min(kStageBytes, bytes - o));
+    hostCopy((char*)host + o, c->stage[k % 2], std::min(part, bytes - o));
     if (k + 2 < chunks) E3D_RET(fetch(k + 2));
   }
   return E3D_OK;

@@ -337,6 +337,7 @@ static int zeroFields(Context* c, Fields9& f, int ncomp = NCOMP) {
 // fault in side by side only across several MB (a Born adjoint call that fetches eight planes of 17 MB:
 // 38.4 against 51.5 ms).  A context starts with the small ones and takes the large ones once the copies it
 // has made would have paid for them: kStageEarned bytes, those out counted four times.
+constexpr size_t kMediumPart = (size_t)32 << 20;  // of a host medium plane at a time; staged copies take it
 constexpr size_t kStageSmall = (size_t)1 << 20, kStageLarge = (size_t)8 << 20, kStageEarned = (size_t)1 << 29;
 
 static bool stageBuffers(Context* c, size_t bytes) {
@@ -556,29 +557,66 @@ double deviceBytesInUse(const Context* c) {
   return (double)(total - free);
 }
 
+// `rows` unpadded rows on the device into the context's rows at dst.  A kernel of its own: strided
+// cudaMemcpy2DAsync copies took twice the time of whole ones (a medium of 392x392x388 cells: 1.29 ms, 0.78 so).
+static int spreadRows(Context* c, const float* src, float* dst, long long rows) {
+  const int nz = c->d.nz, pz = c->g.pz;
+  const unsigned grid = (unsigned)std::min<long long>((rows + 7) / 8, (long long)c->numSMs * 16);
+  if (nz % 4 == 0 && (uintptr_t)src % 16 == 0)
+    kSpreadRows<float4><<<grid, 256, 0, c->st>>>((const float4*)src, (float4*)dst, nz / 4, pz / 4, rows);
+  else
+    kSpreadRows<float><<<grid, 256, 0, c->st>>>(src, dst, nz, pz, rows);
+  E3D_LAUNCH_CHECK();
+  return E3D_OK;
+}
+
+// One medium plane into the context's rows, from the host in parts of whole rows through the scratch.
+static int mediumPlane(Context* c, const float* src, float* dst, bool onDevice) {
+  const size_t bytes = (size_t)c->cells * sizeof(float), row = (size_t)c->d.nz * sizeof(float);
+  const long long rows = (long long)c->d.nx * c->d.ny;
+  if (c->g.pz == c->d.nz) {
+    if (!onDevice) return copyIn(c, dst, src, bytes);
+    E3D_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, c->st));
+    return E3D_OK;
+  }
+  if (onDevice) return spreadRows(c, src, dst, rows);
+  const long long part = std::min<long long>(rows, std::max<long long>(1, (long long)(kMediumPart / row)));
+  for (long long r = 0; r < rows; r += part) {
+    const long long n = std::min(part, rows - r);
+    E3D_RET(copyIn(c, c->scratch, (const char*)src + (size_t)r * row, (size_t)n * row));
+    E3D_RET(spreadRows(c, (const float*)c->scratch, dst + r * c->g.pz, n));
+  }
+  return E3D_OK;
+}
+
 int setMedium(Context* c, const float* const* planes, bool onDevice) {
   E3D_ARG(c && planes, "null argument");
+  for (int k = 0; k < NMED; k++) E3D_ARG(planes[k] != nullptr, "null medium plane");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
-  const size_t bytes = (size_t)c->cells * sizeof(float), row = (size_t)c->d.nz * sizeof(float);
-  for (int k = 0; k < NMED; k++) {
-    E3D_ARG(planes[k] != nullptr, "null medium plane");
-    if (!c->med[k]) E3D_RET(fieldAlloc(c, &c->med[k]));
-    const float* src = planes[k];
-    if (!onDevice && c->g.pz != c->d.nz) {
-      // one copy over the bus, then the rows apart on the device
-      E3D_RET(scratchAtLeast(c, bytes));
-      E3D_RET(copyIn(c, c->scratch, src, bytes));
-      src = (const float*)c->scratch;
+  auto buffers = [&]() -> int {
+    for (int k = 0; k < NMED; k++)
+      if (!c->med[k]) E3D_RET(fieldAlloc(c, &c->med[k]));
+    if (!onDevice && c->g.pz != c->d.nz)
+      E3D_RET(scratchAtLeast(c, std::min((size_t)c->cells * sizeof(float),
+                                         std::max(kMediumPart, (size_t)c->d.nz * sizeof(float)))));
+    return E3D_OK;
+  };
+  int st = buffers();
+  if (st == E3D_ERR_OOM && !c->haveMedium && c->fieldOff != FAT) {
+    // a first medium that has no room in padded rows: unpadded ones from the start
+    for (float*& m : c->med) {
+      fieldFree(c, m);
+      m = nullptr;
     }
-    if (c->g.pz != c->d.nz)
-      E3D_CUDA_TRY(cudaMemcpy2DAsync(c->med[k], (size_t)c->g.pz * sizeof(float), src, row, row,
-                                     (size_t)c->d.nx * c->d.ny, cudaMemcpyDeviceToDevice, c->st));
-    else if (onDevice)
-      E3D_CUDA_TRY(cudaMemcpyAsync(c->med[k], src, bytes, cudaMemcpyDeviceToDevice, c->st));
-    else
-      E3D_RET(copyIn(c, c->med[k], src, bytes));
+    E3D_RET(dropFields(c));
+    setUnpadded(c);
+    st = buffers();
   }
-  E3D_CUDA_TRY(cudaStreamSynchronize(c->st));
+  E3D_RET(st);
+  for (int k = 0; k < NMED && st == E3D_OK; k++) st = mediumPlane(c, planes[k], c->med[k], onDevice);
+  const cudaError_t e = cudaStreamSynchronize(c->st);  // the caller's planes are read, whatever happened
+  E3D_RET(st);
+  E3D_CUDA_TRY(e);
   c->haveMedium = true;
   c->ckptValid = false;
   c->tailValid = false;

@@ -57,6 +57,19 @@ __device__ __forceinline__ long long cellIndex(const GridConst& g, long long pos
   return g.pz == g.nz ? pos : pos / g.nz * g.pz + pos % g.nz;
 }
 
+// Rows of nz values in unpadded rows (src) to rows of pitch pz (dst), a warp per row.
+template <typename V>
+__global__ void __launch_bounds__(256) kSpreadRows(const V* __restrict__ src, V* __restrict__ dst, int nz, int pz,
+                                                   long long rows) {
+  const int lane = threadIdx.x & 31;
+  for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
+    const V* a = src + r * nz;
+    V* b = dst + r * pz;
+#pragma unroll 4
+    for (int z = lane; z < nz; z += 32) b[z] = a[z];
+  }
+}
+
 // Medium-premultiplied wavefield at one cell (stepAdjGpuBorn_3D, kernelsElaGpu_3D.cu:864-920).
 __device__ __forceinline__ void premultiply(const float* v, float rhox, float rhoy, float rhoz, float l2m, float lam,
                                             float muxz, float muxy, float muyz, float* q) {

@@ -193,3 +193,47 @@ def test_staged_planes_in_and_out():
         init = [rng.standard_normal((ny, nx, nz), dtype=np.float32) for _ in range(8)]
         _equal(pr.born_adjoint(sig, dat, spos, rpos, init), init)
     pr.close()
+
+
+@pytest.mark.parametrize("nz,nx,ny", [(16, 9, 10), (17, 13, 11), (72, 40, 20), (101, 30, 21), (168, 200, 188)])
+def test_medium_from_host_and_device(nz, nx, ny):
+    """The medium from host planes, from device planes and from device planes off the 16-byte grid gives
+    the same traces (rows below and above a warp, of every remainder mod 4, one part and several)."""
+    nts = 4
+    rng = np.random.default_rng(9)
+    med = _medium(nz, nx, ny)
+    sp, so, rp, ro, sig = _device_sets(rng, nz, nx, ny, nts)
+    flat = torch.empty(med.size + 1, device="cuda")
+    off = flat[1:].view(med.shape)
+    off.copy_(torch.from_numpy(med))
+    out = []
+    for m in (med, torch.from_numpy(med).cuda(), off):
+        torch.cuda.synchronize()
+        pr = _propagator(nz, nx, ny, nts)
+        pr.set_medium(m)
+        rec = torch.empty((nts, ro[9]), device="cuda")
+        pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
+        pr.synchronize()
+        out.append(rec.cpu().numpy())
+        pr.close()
+    assert np.abs(out[0]).max() > 0
+    _equal(out[1:], [out[0]] * 2)
+
+
+def test_first_medium_fits_without_padding():
+    """Memory for the medium's planes in unpadded rows only (72-cell rows: a third more when padded)."""
+    nz, nx, ny, nts = 72, 200, 400, 4
+    rng = np.random.default_rng(10)
+    med = _medium(nz, nx, ny)
+    sp, so, rp, ro, sig = _device_sets(rng, nz, nx, ny, nts)
+    out = []
+    for short in (False, True):
+        pr = _propagator(nz, nx, ny, nts)
+        with _memory_left(9.5 * 4 * nz * nx * ny) if short else contextlib.nullcontext():
+            pr.set_medium(med)
+        rec = torch.empty((nts, ro[9]), device="cuda")
+        pr.nl_propagate_device(False, sp, so, rp, ro, sig, rec)
+        pr.synchronize()
+        out.append(rec.cpu().numpy())
+        pr.close()
+    np.testing.assert_array_equal(out[1], out[0])

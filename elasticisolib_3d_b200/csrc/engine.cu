@@ -2299,6 +2299,9 @@ static Fields9& ringAt(std::vector<Fields9>& r, long long m) {
   return r[(size_t)(((m % R) + R) % R)];
 }
 
+// Whether every level of a ring has its memory.
+static bool ringComplete(const std::vector<Fields9>& ring) { return !ring.empty() && ring.back().p[NCOMP - 1]; }
+
 // Allocate a ring of `levels` levels whose first two are a and b; levels -1 and 0 zeroed.  The cells
 // around the updated ones read as zero in every level: no step writes them, and a slab run, which
 // does, leaves `ghosts` set.
@@ -2306,15 +2309,13 @@ static int ensureRing(Context* c, std::vector<Fields9>& ring, Fields9& a, Fields
   if (ring.empty()) {
     E3D_RET(allocFields(c, a, false));
     E3D_RET(allocFields(c, b, false));
-    ring.push_back(a);
-    ring.push_back(b);
-    while ((int)ring.size() < levels) {
-      Fields9 f;
-      E3D_RET(allocFields(c, f, false));
-      ring.push_back(f);
-    }
+    ring.assign(levels, Fields9{});
+    ring[0] = a;
+    ring[1] = b;
   }
   E3D_ARG((int)ring.size() == levels, "ring size changed");
+  // levels a call before this one had no memory for are made now
+  for (auto& f : ring) E3D_RET(allocFields(c, f, false));
   if (c->ghosts && &ring == &c->adjRing) {
     for (auto& f : ring) E3D_RET(zeroFields(c, f));
     c->ghosts = false;
@@ -2500,7 +2501,7 @@ static int bornForwardDevice(Context* c, const DevSignals& srcSet, const DevSign
   // with a ring of source levels one launch per block decimates them and the steps carry no
   // accumulators (188 -> 140 B per cell and step)
   bool ring = ringLevels(c) > 0;
-  if (ring && c->srcRing.empty()) {
+  if (ring && !ringComplete(c->srcRing)) {
     // the ring's levels beside the two kept, if the device has the memory for them and the rest of the pass
     size_t free = 0, total = 0;
     E3D_CUDA_TRY(cudaMemGetInfo(&free, &total));
@@ -2627,7 +2628,7 @@ static double pendingAdjointBytes(const Context* c, long long n) {
   const int R = ringLevels(c);
   if (R) {
     // the adjoint ring (w0, w1 and R-2 more levels) and the carried decimation
-    if (c->adjRing.empty()) b += (double)(R - 2) * NCOMP * f + (c->w0.p[0] ? 0 : 18 * f);
+    if (!ringComplete(c->adjRing)) b += (double)(R - 2) * NCOMP * f + (c->w0.p[0] ? 0 : 18 * f);
     if (!c->ss[0].p[0]) b += NCOMP * f;
   } else {
     if (!c->w0.p[0]) b += 18 * f;

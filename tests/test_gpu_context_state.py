@@ -237,3 +237,48 @@ def test_first_medium_fits_without_padding():
         out.append(rec.cpu().numpy())
         pr.close()
     np.testing.assert_array_equal(out[1], out[0])
+
+
+def _gradient(pr, sets, nts, ny, nx, nz, short=None):
+    """Predicted traces and gradient planes of the traces themselves; short: memory left for the
+    gradient pass."""
+    sp, so, rp, ro, sig = sets
+    rec = torch.empty((nts, ro[9]), device="cuda")
+    grad = torch.zeros((8, ny, nx, nz), device="cuda")
+    pr.fwi_forward_device(sp, so, rp, ro, sig, rec)
+    pr.synchronize()
+    with _memory_left(short) if short else contextlib.nullcontext():
+        pr.fwi_gradient_device(sp, so, rp, ro, sig, rec, grad)
+        pr.synchronize()
+    return rec.cpu().numpy(), grad.cpu().numpy()
+
+
+def test_gradient_after_a_forward_that_ran_out_of_memory():
+    """A checkpointed forward that found no memory for all its levels leaves what it got to the next,
+    which runs once there is more."""
+    nz, nx, ny, nts = 72, 200, 400, 6
+    rng = np.random.default_rng(11)
+    med = _medium(nz, nx, ny)
+    sets = _device_sets(rng, nz, nx, ny, nts)
+    out = []
+    for short in (False, True):
+        pr = _propagator(nz, nx, ny, nts)
+        pr.set_medium(med)
+        pr.set_checkpoint_policy("fp32", 2)
+        pr.set_velocity_storage("fp32")
+        if short:
+            sp, so, rp, ro, sig = sets
+            rec = torch.empty((nts, ro[9]), device="cuda")
+            pr.synchronize()
+            with _memory_left(24 * 4 * nz * nx * ny):
+                with pytest.raises(N.E3DError, match="memory"):
+                    pr.fwi_forward_device(sp, so, rp, ro, sig, rec)
+                torch.cuda.synchronize()
+                held = torch.cuda.mem_get_info()[0]
+                with pytest.raises(N.E3DError, match="memory"):
+                    pr.fwi_forward_device(sp, so, rp, ro, sig, rec)
+                torch.cuda.synchronize()
+                assert torch.cuda.mem_get_info()[0] >= held
+        out.append(_gradient(pr, sets, nts, ny, nx, nz))
+        pr.close()
+    _equal(out[1], out[0])

@@ -3433,12 +3433,16 @@ int fwiGradientDevice(Context* c, const DevSignals& srcSet, const DevSignals& re
   E3D_ARG(c && c->haveMedium, "medium not set");
   E3D_ARG(pert8 != nullptr, "null gradient planes");
   E3D_RET(rejectFreeSurface(c));
+  E3D_ARG(c->ckptValid, "no checkpoints for this shot");
+  for (int k = 0; k < NMED; k++) E3D_ARG(pert8[k] != nullptr, "null gradient plane");
   E3D_CUDA_TRY(cudaSetDevice(c->d.device));
-  for (int k = 0; k < NMED; k++) {
-    E3D_ARG(pert8[k] != nullptr, "null gradient plane");
-    c->pertDev[k] = pert8[k];  // accumulate straight into the caller's planes
-  }
-  int st = adjointPassFromCheckpoints(c, srcSet, recSet, srcSig, residual, map, srcAdj);
+  for (int k = 0; k < NMED; k++) c->pertDev[k] = pert8[k];  // accumulate straight into the caller's planes
+  // a pass in unpadded rows, after memory ran out in padded ones, makes its checkpoints again: every
+  // buffer is allocated before the gradient planes are touched
+  int st = withRows(c, [&]() -> int {
+    if (!c->ckptValid) E3D_RET(sourcePassWithCheckpoints(c, srcSet, nullptr, srcSig, nullptr, nullptr));
+    return adjointPassFromCheckpoints(c, srcSet, recSet, srcSig, residual, map, srcAdj);
+  });
   for (int k = 0; k < NMED; k++) c->pertDev[k] = nullptr;
   return st;
 }

@@ -282,3 +282,22 @@ def test_gradient_after_a_forward_that_ran_out_of_memory():
         out.append(_gradient(pr, sets, nts, ny, nx, nz))
         pr.close()
     _equal(out[1], out[0])
+
+
+def test_gradient_fits_without_padding():
+    """A gradient whose forward had room for padded rows and which has room for its own fields in
+    unpadded ones only (72-cell rows: a third more when padded): the planes of one with the room."""
+    nz, nx, ny, nts, sub = 72, 200, 400, 6, 4
+    rng = np.random.default_rng(12)
+    med = _medium(nz, nx, ny)
+    sets = _device_sets(rng, nz, nx, ny, nts)
+    out = []
+    for short in (None, 1.15 * (sub + 2) * 9 * 4 * nz * nx * ny):  # the adjoint ring and a carried block
+        pr = _propagator(nz, nx, ny, nts, sub)
+        pr.set_medium(med)
+        pr.set_checkpoint_policy("fp32", 2)
+        pr.set_velocity_storage("fp32")
+        out.append(_gradient(pr, sets, nts, ny, nx, nz, short))
+        pr.close()
+    assert np.abs(out[0][1]).max() > 0
+    _equal(out[1], out[0])

@@ -2043,8 +2043,11 @@ int nlPropagateSlabsHost(Context* const* slabs, int nSlabs, int nyGlobal, bool a
     if (st == E3D_OK) st = stageSlabTables(c, r.pos[1], r.R);
     if (st == E3D_OK) st = adjoint ? stageSignalsZero(c, r.S) : stageSignalsIn(c, r.S, in);
     if (st == E3D_OK) st = adjoint ? stageSignalsIn(c, r.R, in) : stageSignalsZero(c, r.R);
-    if (st == E3D_OK) st = allocFields(c, c->w0, true);
-    if (st == E3D_OK) st = allocFields(c, c->w1, true);
+    if (st == E3D_OK)
+      st = withRows(c, [&]() -> int {
+        E3D_RET(allocFields(c, c->w0, true));
+        return allocFields(c, c->w1, true);
+      });
     c->ghosts = true;
     c->tailReady = takesTail(c);
     c->pending = {};
@@ -2130,9 +2133,7 @@ int nlPropagateSlabsHost(Context* const* slabs, int nSlabs, int nyGlobal, bool a
   return st;
 }
 
-int stepOnly(Context* c, int mode, int nSteps) {
-  E3D_ARG(c && c->haveMedium, "medium not set");
-  E3D_ARG(mode >= 0 && mode <= 5, "bad mode");
+static int stepPass(Context* c, int mode, int nSteps) {
   // modes 3..5: modes 0..2 with the new level decimated into two coarse
   // accumulators, as the fused-accumulator passes run them (3 velocity fields for
   // the source recompute, 9 fields for the adjoint).  The ring passes' exact
@@ -2172,6 +2173,12 @@ int stepOnly(Context* c, int mode, int nSteps) {
     if (dual) swapF(c->q0, c->q1);
   }
   return E3D_OK;
+}
+
+int stepOnly(Context* c, int mode, int nSteps) {
+  E3D_ARG(c && c->haveMedium, "medium not set");
+  E3D_ARG(mode >= 0 && mode <= 5, "bad mode");
+  return withRows(c, [&] { return stepPass(c, mode, nSteps); });
 }
 
 int checkpointSegment(const Context* c) { return c->ckptSegLen; }

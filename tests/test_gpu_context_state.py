@@ -301,3 +301,35 @@ def test_gradient_fits_without_padding():
         pr.close()
     assert np.abs(out[0][1]).max() > 0
     _equal(out[1], out[0])
+
+
+@pytest.mark.parametrize("what", ["slabs", "steps"])
+def test_levels_fit_without_padding(what):
+    """Slab runs and bare steps with room for their two levels in unpadded rows only (72-cell rows: a
+    third more when padded)."""
+    nz, nx, ny, nts = 72, 200, 400, 4
+    rng = np.random.default_rng(13)
+    med = _medium(nz, nx, ny)
+    left = 1.15 * 18 * 4 * nz * nx * ny
+    if what == "steps":
+        pr = _propagator(nz, nx, ny, nts)
+        pr.set_medium(med)
+        pr.synchronize()
+        with _memory_left(left):
+            pr.step_only(0, 2)
+            pr.synchronize()
+        pr.close()
+        return
+    spos = [_points(rng, nz, nx, ny, 4) for _ in range(7)]
+    rpos = [np.unique(np.concatenate([p, _points(rng, nz, nx, ny, 60)])) for p in spos]
+    model = random_signals(spos, nts, rng)
+    out = []
+    for short in (False, True):
+        sl = _propagator(nz, nx, ny, nts, cls=SlabPropagator, devices=(0, 0))
+        sl.set_medium(med)
+        torch.cuda.synchronize()
+        with _memory_left(left) if short else contextlib.nullcontext():
+            out.append(sl.nl_forward(model, spos, rpos))
+        sl.close()
+    assert max(np.abs(x).max() for x in out[0]) > 0
+    _equal(out[1], out[0])

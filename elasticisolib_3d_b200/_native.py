@@ -55,6 +55,7 @@ SIGNATURES = {
     "e3d_stream": ([P], P),
     "e3d_set_stream": ([P, P, I], I),
     "e3d_cells_per_step": ([P], LL),
+    "e3d_field_cells": ([P], LL),
     "e3d_checkpoint_segment": ([P], I),
     "e3d_nl_forward": ([P] * 7, I),
     "e3d_nl_adjoint": ([P] * 7, I),

@@ -368,6 +368,8 @@ int e3d_set_stream(e3d_context* ctx, void* s, int use_own) {
   return setStream(ctx->c, (cudaStream_t)s, use_own != 0);
 }
 
+long long e3d_field_cells(const e3d_context* ctx) { return (ctx && ctx->c) ? fieldCells(ctx->c) : 0; }
+
 long long e3d_cells_per_step(const e3d_context* ctx) { return (ctx && ctx->c) ? cellsPerStep(ctx->c) : 0; }
 
 int e3d_checkpoint_segment(const e3d_context* ctx) { return (ctx && ctx->c) ? checkpointSegment(ctx->c) : 0; }

@@ -548,6 +548,7 @@ int setStream(Context* c, cudaStream_t s, bool useOwn) {
   c->st = useOwn ? c->own : s;
   return E3D_OK;
 }
+long long fieldCells(const Context* c) { return c->g.n; }
 long long cellsPerStep(const Context* c) {
   return (long long)(c->d.nz - 2 * FAT) * (c->d.nx - 2 * FAT) * (c->d.ny - 2 * FAT);
 }

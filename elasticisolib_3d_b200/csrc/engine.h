@@ -136,6 +136,7 @@ size_t staticWorkBytes();
 // Timing/inspection helpers
 int stepOnly(Context* c, int mode, int nSteps);  // run nSteps bare steps on the working state
 long long cellsPerStep(const Context* c);
+long long fieldCells(const Context* c);  // cells of a field as the context holds it (padded rows)
 int checkpointSegment(const Context* c);  // coarse blocks per checkpoint segment (0 before first use)
 double deviceBytesInUse(const Context* c);
 cudaStream_t stream(Context* c);

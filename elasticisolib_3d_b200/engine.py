@@ -44,9 +44,9 @@ def domain_decomposition(ny, n_gpu, fat=None, min_pad=0):
 
 def forward_batch_plan(n_shots, n_cells, nts, src_points, rec_points, free_bytes, margin=0.9):
     """Shots per batched forward launch admitted by device memory: each shot of a batch holds both
-    leapfrog levels of the nine fields (18 * n_cells floats), its time-major source and receiver
-    signals (nts * (src_points + rec_points) floats) and its position tables (8 B per point);
-    at most `margin` of `free_bytes` is used.  Returns the batches as lists of shot indices, as
+    leapfrog levels of the nine fields (18 * n_cells floats, n_cells as Propagator.field_cells), its
+    time-major source and receiver signals (nts * (src_points + rec_points) floats) and its position
+    tables (8 B per point); at most `margin` of `free_bytes` is used.  Returns the batches as lists of shot indices, as
     even in size as the budget allows.  ValueError when not even one shot fits."""
     if n_shots < 1:
         return []
@@ -241,6 +241,11 @@ class Propagator:
         return int(N.lib().e3d_checkpoint_segment(self._h))
 
     @property
+    def field_cells(self):
+        """Cells of one field as the context holds it (nz*nx*ny, or more in padded rows)."""
+        return int(N.lib().e3d_field_cells(self._h))
+
+    @property
     def cells_per_step(self):
         return int(N.lib().e3d_cells_per_step(self._h))
 
@@ -317,8 +322,11 @@ class Propagator:
             free_bytes, _ = torch.cuda.mem_get_info(torch.device("cuda", self.device))
         src_points = max(sum(len(sp[COMP_GRID[k]]) for k in range(9)) for sp in src_pos7s) if src_pos7s else 0
         rec_points = sum(len(rec_pos7[COMP_GRID[k]]) for k in range(9))
-        plan = forward_batch_plan(len(models), self.nz * self.nx * self.ny, self.nts, src_points, rec_points,
-                                  free_bytes, margin)
+        args = (self.nts, src_points, rec_points, free_bytes, margin)
+        try:
+            plan = forward_batch_plan(len(models), self.field_cells, *args)
+        except ValueError:  # not one shot in padded rows: a batch gives the padding up
+            plan = forward_batch_plan(len(models), self.nz * self.nx * self.ny, *args)
         out = []
         for batch in plan:
             out.extend(self.nl_forward_batch([models[i] for i in batch], [src_pos7s[i] for i in batch], rec_pos7))
@@ -350,7 +358,8 @@ class Propagator:
                 for k in range(8)]
         SP, SN, k1 = _geom(src_pos7)
         RP, RN, k2 = _geom(rec_pos7)
-        N.call("e3d_born_image" if fresh else "e3d_born_adjoint", self._h, N.ptr_array(src), N.ptr_array(data), SP, SN, RP, RN, N.ptr_array(pert))
+        N.call("e3d_born_image" if fresh else "e3d_born_adjoint", self._h, N.ptr_array(src), N.ptr_array(data), SP, SN,
+               RP, RN, N.ptr_array(pert))
         return pert
 
     def kernel_timing(self, every):

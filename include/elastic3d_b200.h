@@ -318,6 +318,10 @@ void* e3d_stream(e3d_context* ctx);
 int e3d_set_stream(e3d_context* ctx, void* stream, int use_own);
 /* Updated cells per fine step ((nz-8)(nx-8)(ny-8)). */
 long long e3d_cells_per_step(const e3d_context* ctx);
+/* Cells of one field as the context holds it: rows are padded to a multiple of
+ * 32 floats while the fields take a small part of the device's memory, and
+ * padding is given up where a pass has no room for it. */
+long long e3d_field_cells(const e3d_context* ctx);
 /* Coarse blocks per checkpoint segment chosen by the last checkpointed forward (0 before). */
 int e3d_checkpoint_segment(const e3d_context* ctx);
 /* Storage of the decimated source velocity kept per segment for the imaging
@@ -431,7 +435,7 @@ int e3d_nl_propagate_device(e3d_context* ctx, int adjoint, const long long* src_
  * range off10[k]..off10[k+1] holds the entries of every shot, and an entry of
  * shot s carries s*nz*nx*ny added to its grid position.  Signals are
  * time-major over the combined tables.  The shots' wavefields take
- * 18*shots*nz*nx*ny floats; nz % 4 == 0; no free surface.  The tables are
+ * 18*shots*e3d_field_cells floats; nz % 4 == 0; no free surface.  The tables are
  * checked on the device first, as above, against the stacked grids. */
 int e3d_nl_forward_batch_device(e3d_context* ctx, int shots, const long long* src_pos_dev, const int* src_off10,
                                 const long long* rec_pos_dev, const int* rec_off10, const float* src_sig_dev,

@@ -333,3 +333,27 @@ def test_levels_fit_without_padding(what):
         sl.close()
     assert max(np.abs(x).max() for x in out[0]) > 0
     _equal(out[1], out[0])
+
+
+def test_admitted_shots_leave_the_rows():
+    """Shots dealt into batches by the free memory fit in the rows the context has."""
+    nz, nx, ny, nts, shots = 72, 200, 200, 3, 10
+    rng = np.random.default_rng(14)
+    spos = [[_points(rng, nz, nx, ny, 4) for _ in range(7)] for _ in range(shots)]
+    rpos = [_points(rng, nz, nx, ny, 50) for _ in range(7)]
+    models = [random_signals(sp, nts, rng) for sp in spos]
+    pr = _propagator(nz, nx, ny, nts, q2compat=0)
+    pr.set_medium(_medium(nz, nx, ny))
+    cells = pr.field_cells
+    assert cells == 96 * nx * ny
+    whole = pr.nl_forward_batch(models, spos, rpos)
+    pr.close()
+    pr = _propagator(nz, nx, ny, nts, q2compat=0)
+    pr.set_medium(_medium(nz, nx, ny))
+    pr.synchronize()
+    with _memory_left(1.1 * shots * 18 * 4 * nz * nx * ny + (64 << 20)):
+        dealt = pr.nl_forward_shots(models, spos, rpos)
+    assert pr.field_cells == cells
+    for a, b in zip(dealt, whole):
+        _equal(a, b)
+    pr.close()

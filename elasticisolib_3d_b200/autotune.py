@@ -2,8 +2,9 @@
 
 Candidates are the (x tile width, pipeline stages, loader) forms the engine builds, timed with
 CUDA events on the context's stream over a few bare steps of the mode that will dominate
-(0 forward / 1 time-reversed / 2 the FWI adjoint: exact transpose on the dual state).  Variants
-the grid cannot run (cp.async and TMA need nz % 4 == 0) are skipped.  The working wavefields of the context are overwritten; call it before propagating.
+(0 forward / 1 time-reversed / 2 the FWI adjoint: exact transpose on the dual state).  Every
+variant runs on every grid.  The working wavefields of the context are overwritten; call it before
+propagating.
 The y-chunking of the stepper grid stays automatic (a measured per-mode rule in the engine).
 """
 from __future__ import annotations
@@ -22,8 +23,6 @@ def autotune(prop: Propagator, mode: int = 0, steps: int = 6, warmup: int = 2, c
     """Time each candidate on `prop`'s grid, select the fastest and return
     (best, {variant: ms_per_step}).  The medium must be set."""
     cands = list(candidates or CANDIDATES)
-    if prop.nz % 4 != 0:
-        cands = [c for c in cands if c[2] == "plain"]
     if mode in (2, 5):
         # the dual-state adjoint runs on the TMA steppers only
         cands = [c for c in cands if c[2] in TMA_LOADERS]
@@ -52,10 +51,6 @@ def autotune_gradient(prop: Propagator, steps: int = 4, warmup: int = 2):
     (mode 2): minimises 2*t0 + t2 over the TMA candidates (the dual adjoint runs on TMA only).
     Returns (best, {variant: (t0, t2)})."""
     cands = [c for c in CANDIDATES if c[2] in TMA_LOADERS]
-    if prop.nz % 4 != 0:
-        # no TMA form fits the grid; the plain stepper runs every pass
-        prop.set_stepper_variant(8, 2, "plain")
-        return (8, 2, "plain"), {}
     per = {}
     for mode in (0, 2):
         _, t = autotune(prop, mode, steps, warmup, cands)

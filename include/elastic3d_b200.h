@@ -284,7 +284,8 @@ int e3d_set_medium(e3d_context* ctx, const float* const* planes8, int on_device)
  * 6 TMA with the velocity and stress updates of a step as two CTA roles of one
  * launch, 8-wide tiles, 7 the same for the forward and time-reversed steps with
  * the exact adjoint on loader 2's stepper, 8 as 7 with each thread updating two
- * consecutive z cells from paired shared-memory loads; 1 to 8 need nz % 4 == 0). */
+ * consecutive z cells from paired shared-memory loads).  Every loader runs on
+ * every grid: fields are held in rows of whole 16-byte words. */
 int e3d_set_stepper_variant(e3d_context* ctx, int tx, int stages, int loader);
 /* Nonlinear propagation (e3d_nl_* and the seam's propElastic*Gpu_3D): on = 1
  * (default) captures one coarse block as a CUDA graph after running the first
@@ -344,8 +345,8 @@ int e3d_set_decimation_ring(e3d_context* ctx, int on);
 /* y chunks of the block imaging launch of the decimation ring (0 = automatic:
  * the rule of the stepper grids).  A tuning knob; no counterpart in the reference. */
 int e3d_set_imaging_chunks(e3d_context* ctx, int chunks);
-/* Kernel of that block imaging: 0 = automatic (2 where the TMA forms apply:
- * nz % 4 == 0 and a TMA stepper loader, else 1), 1 = one thread per cell
+/* Kernel of that block imaging: 0 = automatic (2 with a TMA stepper
+ * loader, else 1), 1 = one thread per cell
  * reading every operand from global memory, 2 = y-march with the velocity
  * tiles staged by TMA and the adjoint levels read per cell, 3 = y-march with
  * the velocity tiles, the adjoint levels and the medium staged by TMA (one

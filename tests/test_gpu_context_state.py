@@ -357,3 +357,35 @@ def test_admitted_shots_leave_the_rows():
     for a, b in zip(dealt, whole):
         _equal(a, b)
     pr.close()
+
+
+@pytest.mark.parametrize("surface", [0, 1])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_slabs_of_unlike_rows_equal_the_whole_grid(adjoint, surface):
+    """Slabs of one grid, the first of which gave up its rows' padding: the traces of the undivided
+    grid, with the free surface (applied in the stepper) too."""
+    nz, nx, ny, nts = 72, 120, 300, 5
+    rng = np.random.default_rng(15)
+    med = _medium(nz, nx, ny)
+    spos = [_points(rng, nz, nx, ny, 20) for _ in range(7)]
+    rpos = [np.unique(np.concatenate([p, _points(rng, nz, nx, ny, 400)])) for p in spos]
+    whole = _propagator(nz, nx, ny, nts, free_surface=surface)
+    whole.set_medium(med)
+    sl = _propagator(nz, nx, ny, nts, cls=SlabPropagator, devices=(0, 0), free_surface=surface)
+    sl.set_medium(med)
+    first, n0 = sl.slabs[0], nz * nx * sl.sizes[0]
+    first.synchronize()
+    with _memory_left(1.15 * 18 * 4 * n0):
+        first.step_only(0, 1)
+        first.synchronize()
+    assert first.field_cells == n0 and sl.slabs[1].field_cells > nz * nx * sl.sizes[1]
+    if adjoint:
+        dat = random_signals(rpos, nts, rng)
+        got, ref = sl.nl_adjoint(dat, spos, rpos), whole.nl_adjoint(dat, spos, rpos)
+    else:
+        sig = random_signals(spos, nts, rng)
+        got, ref = sl.nl_forward(sig, spos, rpos), whole.nl_forward(sig, spos, rpos)
+    assert max(np.abs(x).max() for x in ref) > 0
+    _equal(got, ref)
+    sl.close()
+    whole.close()

@@ -110,6 +110,71 @@ def test_padded_rows_give_way_to_memory():
             np.testing.assert_array_equal(x, y)
 
 
+ODD = [(29, 21, 19, 8, 3), (45, 24, 31, 6, 4), (31, 20, 26, 7, 2)]
+LOADERS = [(8, 2, "plain"), (16, 2, "plain"), (8, 2, "cpasync"), (16, 2, "cpasync"), (8, 3, "cpasync"), (8, 2, "tma"),
+           (16, 2, "tma"), (8, 3, "tma"), (8, 2, "tma-ring"), (8, 2, "tma-ring-ldg"), (8, 2, "tma-ring-ldg2"),
+           (8, 2, "split"), (8, 3, "split"), (8, 4, "split"), (8, 3, "split-fwd"), (8, 2, "split-pair"),
+           (8, 4, "split-pair")]
+
+
+def _odd_case(nz, nx, ny, nts, sub):
+    rng = np.random.default_rng(nz)
+    el = S.elastic_from_velocity(*S.gaussian_perturbed_model((ny, nx, nz), 2500.0, 1443.0, 2000.0, 0.1, 2.0, 5))
+    dts = 0.0005 * sub
+    med = O.medium_planes(el, dts / sub, np.float32)
+    p = O.PropParams(nz, nx, ny, nts, sub, 3, 10.0, 10.0, 10.0, dts)
+    spos = [_points(rng, nz, nx, ny, 4) for _ in range(7)]
+    rpos = [_points(rng, nz, nx, ny, 50) for _ in range(7)]
+    pr = Propagator(nz, nx, ny, nts, sub, 3, 10.0, 10.0, 10.0, dts)
+    pr.set_medium(med)
+    return rng, p, med.astype(np.float64), spos, rpos, pr
+
+
+@pytest.mark.parametrize("nz,nx,ny,nts,sub", ODD)
+def test_every_stepper_on_odd_rows(nz, nx, ny, nts, sub):
+    """The stepper forms that once took rows of a multiple of four cells only, on rows that are not."""
+    rng, p, med, spos, rpos, pr = _odd_case(nz, nx, ny, nts, sub)
+    sig, dat = random_signals(spos, nts, rng), random_signals(rpos, nts, rng)
+    fwd = O.nl_forward_reg(p, med, [s.astype(np.float64) for s in sig], spos, rpos, np.float64)
+    adj = O.nl_adjoint_reg(p, med, [d.astype(np.float64) for d in dat], spos, rpos, np.float64)
+    for v in LOADERS:
+        pr.set_stepper_variant(*v)
+        assert rel_l2(pr.nl_forward(sig, spos, rpos), fwd) < 1e-5, v
+        assert rel_l2(pr.nl_adjoint(dat, spos, rpos), adj) < 1e-5, v
+    pr.close()
+
+
+@pytest.mark.parametrize("nz,nx,ny,nts,sub", ODD)
+def test_image_forms_on_odd_rows(nz, nx, ny, nts, sub):
+    """The Born adjoint on such rows with every imaging kernel, adjoint state, decimation and storage
+    (FP16 states and slots within the 1e-3 that they are allowed on other grids)."""
+    rng, p, med, spos, rpos, pr = _odd_case(nz, nx, ny, nts, sub)
+    sig, dat = random_signals(spos, nts, rng), random_signals(rpos, nts, rng)
+    ref = O.born_adjoint_reg(p, med, [s.astype(np.float64) for s in sig], [d.astype(np.float64) for d in dat], spos,
+                             rpos, None, np.float64)
+
+    def check(bound, **how):
+        pr.set_stepper_variant(*how.get("variant", (8, 3, "split-pair")))
+        pr.set_premultiplied_adjoint(how.get("prem", True))
+        pr.set_decimation_ring(how.get("ring", True))
+        pr.set_imaging_variant(how.get("imaging", "auto"))
+        pr.set_checkpoint_policy(how.get("store", "fp32"), how.get("segment", 3))
+        pr.set_velocity_storage(how.get("store", "fp32"))
+        assert rel_l2(pr.born_adjoint(sig, dat, spos, rpos), ref) < bound, how
+
+    for imaging in ("cells", "tma", "tma-levels", "tma-levels-4"):
+        for prem in (True, False):
+            check(1e-5, imaging=imaging, prem=prem)
+    for variant in ((8, 2, "plain"), (8, 2, "cpasync"), (8, 2, "tma"), (16, 2, "tma"), (8, 3, "split"),
+                    (8, 3, "split-fwd")):
+        check(1e-5, variant=variant)
+        check(1e-5, variant=variant, ring=False)
+    check(1e-5, ring=False)
+    check(1e-3, store="fp16", segment=2)
+    check(1e-3, store="fp16", segment=2, ring=False)
+    pr.close()
+
+
 def test_autotuner_takes_a_fast_stepper_on_odd_rows():
     """Rows of an odd number of cells run every stepper: the plain one, three times slower than the
     default on such a grid, is not what the autotuner picks."""

@@ -188,9 +188,9 @@ static void devFree(Context* c, void* p) {
 // updated cell (z = FAT) and every 32-cell tile row after it are whole 128-byte lines; in unpadded rows
 // a tile row starts 16 bytes into a sector and each store and box touches one more.  Measured on B200,
 // a forward step: 392x392x388 cells 1478 -> 1354 us, 168x200x188 149.7 -> 135.2; the offset of a
-// sector alone (4 floats, unpadded rows) gives 1410 and 140.9.  It costs 8 to 31 floats a row, which
-// grids holding more than 8 % of the device's memory in levels and medium do without, so that what fits
-// the device fits it still.
+// sector alone (4 floats, unpadded rows) gives 1410 and 140.9.  It costs 0 to 31 floats a row, which
+// grids holding more than 8 % of the device's memory in levels and medium do without, and which a context
+// gives up when a pass or its memory plan has no room for it (withRows, choosePlan).
 static void rowLayout(const ContextDesc& d, size_t deviceBytes, int& pitch, int& offset) {
   const double held = 26.0 * sizeof(float) * d.nz * d.nx * d.ny;
   if (held > 0.08 * (double)deviceBytes) {
@@ -2474,7 +2474,7 @@ static int launchImagingBlock(Context* c, long long mEnd, float* const v[4], boo
     static std::atomic<unsigned long long> configured{0};
     E3D_RET(ensureSmemAttr((const void*)kImagingTma, smem, configured));
     // runs of at least 24 planes where those fill the device, else down to two planes (72x72x64
-    // cells: 16 tiles, 32 CTAs of 28 planes took 74 us, 208 of four take 22)
+    // cells: 16 tiles, 32 CTAs of 28 planes took 74 us, 208 of four take 17)
     const long long tiles = (long long)tiz * tix;
     const int minRun = tiles * std::max(1, nyi / 24) >= 2LL * c->numSMs ? 24 : 2;
     const int chunks0 = c->imgChunks > 0 ? std::min(c->imgChunks, nyi) : chooseChunks(c, tiles, nyi, 2, minRun);

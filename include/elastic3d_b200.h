@@ -384,7 +384,8 @@ int e3d_checkpoint_schedule(int blocks, int segment_len, int* seg_start, int max
  * ckpt_type / velocity_type / segment as in e3d_set_checkpoint_policy and
  * e3d_set_velocity_storage.  Outputs (each may be NULL): the state and slot
  * storage types, the segment length and the plan's bytes.  E3D_ERR_OOM when
- * nothing fits.  No device work. */
+ * nothing fits.  The padding of a context's rows takes no part in the plan.  No
+ * device work. */
 int e3d_checkpoint_plan(long long n_cells, int ny, int nts, double budget_bytes, int ckpt_type, int velocity_type,
                         int segment, int* ckpt_used, int* velocity_used, int* segment_len, double* plan_bytes);
 

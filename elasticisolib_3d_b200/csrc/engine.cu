@@ -22,6 +22,7 @@
 #include <unordered_map>
 
 #include <omp.h>
+#include <sys/mman.h>
 
 #include "engine.h"
 #include "kernels.cuh"
@@ -149,7 +150,6 @@ struct Context {
   // pinned staging of large copies between the device and callers' pageable memory (HostCopy)
   char* stage[2] = {};
   cudaEvent_t stageEv[2] = {};
-  size_t stageBytes = 0, stageMoved = 0;  // size of each buffer; bytes copied through them
   // scratch for transposes / signal staging
   void* scratch = nullptr;
   size_t scratchBytes = 0;
@@ -332,53 +332,37 @@ static int zeroFields(Context* c, Fields9& f, int ncomp = NCOMP) {
 // memory go straight to cudaMemcpyAsync.
 // ---------------------------------------------------------------------------
 //
-// Pinning costs about a millisecond for two buffers of 1 MB and 8 to 12 for two of 8 MB, which move 17 MB
-// in 0.49 ms where the small ones take 0.64, and more so out to untouched pages, which the host threads
-// fault in side by side only across several MB (a Born adjoint call that fetches eight planes of 17 MB:
-// 38.4 against 51.5 ms).  A context starts with the small ones and takes the large ones once the copies it
-// has made would have paid for them: kStageEarned bytes, those out counted four times.
+// The buffers are small, since pinning is slow: two of 1 MB take about a millisecond and move 17 MB over
+// 12 threads in 0.55 ms, two of 8 MB take 8 to 12 (and at times hundreds) and move them in 0.5.
 constexpr size_t kMediumPart = (size_t)32 << 20;  // of a host medium plane at a time; staged copies take it
-constexpr size_t kStageSmall = (size_t)1 << 20, kStageLarge = (size_t)8 << 20, kStageEarned = (size_t)1 << 29;
+constexpr size_t kStageBytes = (size_t)1 << 20;
+constexpr size_t kStageFirst = (size_t)16 << 20, kStageNext = (size_t)4 << 20;  // copies staged without and with buffers
+constexpr int kStageThreads = 12;
 
-static bool stageBuffers(Context* c, size_t bytes) {
-  char* p[2] = {};
+static bool staged(Context* c, const void* host, size_t bytes) {
+  if (bytes < (c->stage[1] ? kStageNext : kStageFirst)) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
+  else if (at.type != cudaMemoryTypeUnregistered) return false;
   for (int i = 0; i < 2; i++) {
     if (!c->stageEv[i] && cudaEventCreateWithFlags(&c->stageEv[i], cudaEventDisableTiming) != cudaSuccess) {
       c->stageEv[i] = nullptr;
       cudaGetLastError();
       return false;
     }
-    if (cudaHostAlloc((void**)&p[i], bytes, cudaHostAllocDefault) != cudaSuccess) {
+    if (!c->stage[i] && cudaHostAlloc((void**)&c->stage[i], kStageBytes, cudaHostAllocDefault) != cudaSuccess) {
+      c->stage[i] = nullptr;
       cudaGetLastError();
-      if (i) cudaFreeHost(p[0]);
       return false;
     }
   }
-  for (int i = 0; i < 2; i++) {
-    if (c->stage[i]) {
-      cudaEventSynchronize(c->stageEv[i]);  // the buffer's last copy
-      cudaFreeHost(c->stage[i]);
-    }
-    c->stage[i] = p[i];
-  }
-  c->stageBytes = bytes;
   return true;
 }
 
-static bool staged(Context* c, const void* host, size_t bytes, bool out) {
-  if (bytes < (c->stageBytes ? kStageLarge / 2 : 2 * kStageLarge)) return false;
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) cudaGetLastError();
-  else if (at.type != cudaMemoryTypeUnregistered) return false;
-  if (!c->stageBytes && !stageBuffers(c, kStageSmall)) return false;
-  // without memory for the large buffers the small ones go on
-  if (c->stageBytes < kStageLarge && c->stageMoved >= kStageEarned && !stageBuffers(c, kStageLarge)) c->stageMoved = 0;
-  c->stageMoved += out ? 4 * bytes : bytes;
-  return true;
-}
+static int stageThreads() { return std::max(1, std::min(kStageThreads, omp_get_num_procs())); }
 
 static void hostCopy(char* dst, const char* src, size_t bytes) {
-  const int n = std::max(1, std::min(8, omp_get_num_procs()));
+  const int n = stageThreads();
   const size_t part = ((bytes + n - 1) / n + 4095) / 4096 * 4096;
 #pragma omp parallel for num_threads(n) schedule(static, 1)
   for (int i = 0; i < n; i++) {
@@ -387,16 +371,35 @@ static void hostCopy(char* dst, const char* src, size_t bytes) {
   }
 }
 
+// Has the pages of a destination made before it is written, on several threads and several huge pages
+// at a time (parts of 1 MB fault one huge page after the other: eight planes of 17 MB took 13 ms more).
+// What the pages hold stays; a kernel without the call leaves the faults to the copies.
+static void touchPages(char* dst, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+  const uintptr_t page = 4096, huge = (uintptr_t)2 << 20;
+  const uintptr_t b = ((uintptr_t)dst + page - 1) / page * page, e = ((uintptr_t)dst + bytes) / page * page;
+  if (e <= b) return;
+  const int n = (int)(e / huge - b / huge + 1), team = stageThreads();
+#pragma omp parallel for num_threads(team) schedule(dynamic, 1)
+  for (int i = 0; i < n; i++) {
+    const uintptr_t h = (b / huge + i) * huge, lo = std::max(b, h), hi = std::min(e, h + huge);
+    if (hi > lo) madvise((void*)lo, hi - lo, MADV_POPULATE_WRITE);
+  }
+#else
+  (void)dst;
+  (void)bytes;
+#endif
+}
+
 // Pageable sources are read when this returns, pinned and registered ones when the stream is.
 static int copyIn(Context* c, void* dev, const void* host, size_t bytes) {
-  if (!staged(c, host, bytes, false)) {
+  if (!staged(c, host, bytes)) {
     E3D_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->st));
     return E3D_OK;
   }
-  const size_t part = c->stageBytes;
   int i = 0;
-  for (size_t o = 0; o < bytes; o += part, i ^= 1) {
-    const size_t n = std::min(part, bytes - o);
+  for (size_t o = 0; o < bytes; o += kStageBytes, i ^= 1) {
+    const size_t n = std::min(kStageBytes, bytes - o);
     E3D_CUDA_TRY(cudaEventSynchronize(c->stageEv[i]));  // the buffer's last copy
     hostCopy(c->stage[i], (const char*)host + o, n);
     E3D_CUDA_TRY(cudaMemcpyAsync((char*)dev + o, c->stage[i], n, cudaMemcpyHostToDevice, c->st));
@@ -407,24 +410,25 @@ static int copyIn(Context* c, void* dev, const void* host, size_t bytes) {
 
 // Staged copies are complete when this returns, the others when the stream is.
 static int copyOut(Context* c, void* host, const void* dev, size_t bytes) {
-  if (!staged(c, host, bytes, true)) {
+  if (!staged(c, host, bytes)) {
     E3D_CUDA_TRY(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, c->st));
     return E3D_OK;
   }
-  const size_t part = c->stageBytes, chunks = (bytes + part - 1) / part;
+  const size_t chunks = (bytes + kStageBytes - 1) / kStageBytes;
   auto fetch = [&](size_t k) -> int {
-    const size_t o = k * part;
-    E3D_CUDA_TRY(cudaMemcpyAsync(c->stage[k % 2], (const char*)dev + o, std::min(part, bytes - o),
+    const size_t o = k * kStageBytes;
+    E3D_CUDA_TRY(cudaMemcpyAsync(c->stage[k % 2], (const char*)dev + o, std::min(kStageBytes, bytes - o),
                                  cudaMemcpyDeviceToHost, c->st));
     E3D_CUDA_TRY(cudaEventRecord(c->stageEv[k % 2], c->st));
     return E3D_OK;
   };
+  touchPages((char*)host, bytes);
   for (int i = 0; i < 2; i++) E3D_CUDA_TRY(cudaEventSynchronize(c->stageEv[i]));
   for (size_t k = 0; k < std::min<size_t>(chunks, 2); k++) E3D_RET(fetch(k));
   for (size_t k = 0; k < chunks; k++) {
-    const size_t o = k * part;
+    const size_t o = k * kStageBytes;
     E3D_CUDA_TRY(cudaEventSynchronize(c->stageEv[k % 2]));
-    hostCopy((char*)host + o, c->stage[k % 2], std::min(part, bytes - o));
+    hostCopy((char*)host + o, c->stage[k % 2], std::min(kStageBytes, bytes - o));
     if (k + 2 < chunks) E3D_RET(fetch(k + 2));
   }
   return E3D_OK;

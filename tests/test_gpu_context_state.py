@@ -180,8 +180,8 @@ def test_rows_do_not_change_the_memory_plan(nz, nx, ny, nts, budget):
 
 
 def test_staged_planes_in_and_out():
-    """Image planes of 17 MB sent and fetched through the staging buffers, small and then large (once
-    half a gigabyte was copied): zero data leaves the caller's planes as they were."""
+    """Image planes of 17 MB sent and fetched through the staging buffers: zero data leaves the caller's
+    planes as they were."""
     nz, nx, ny, nts = 168, 168, 152, 3
     rng = np.random.default_rng(8)
     pr = _propagator(nz, nx, ny, nts, sub=1)
@@ -189,7 +189,7 @@ def test_staged_planes_in_and_out():
     spos = [_points(rng, nz, nx, ny, 4) for _ in range(7)]
     rpos = [_points(rng, nz, nx, ny, 9) for _ in range(7)]
     sig, dat = random_signals(spos, nts, rng), [0 * d for d in random_signals(rpos, nts, rng)]
-    for _ in range(4):
+    for _ in range(2):
         init = [rng.standard_normal((ny, nx, nz), dtype=np.float32) for _ in range(8)]
         _equal(pr.born_adjoint(sig, dat, spos, rpos, init), init)
     pr.close()

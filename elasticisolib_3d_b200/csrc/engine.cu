@@ -330,13 +330,13 @@ static int zeroFields(Context* c, Fields9& f, int ncomp = NCOMP) {
 // every page of a fresh array is also touched for the first time.  Here two pinned buffers
 // alternate between the bus and a memcpy over several host threads.  Small copies and callers' pinned
 // memory go straight to cudaMemcpyAsync.
-// ---------------------------------------------------------------------------
-//
 // The buffers are small, since pinning is slow: two of 1 MB take about a millisecond and move 17 MB over
 // 12 threads in 0.55 ms, two of 8 MB take 8 to 12 (and at times hundreds) and move them in 0.5.
+// ---------------------------------------------------------------------------
 constexpr size_t kMediumPart = (size_t)32 << 20;  // of a host medium plane at a time; staged copies take it
 constexpr size_t kStageBytes = (size_t)1 << 20;
-constexpr size_t kStageFirst = (size_t)16 << 20, kStageNext = (size_t)4 << 20;  // copies staged without and with buffers
+// smallest copy that makes the buffers, and that uses them
+constexpr size_t kStageFirst = (size_t)16 << 20, kStageNext = (size_t)4 << 20;
 constexpr int kStageThreads = 12;
 
 static bool staged(Context* c, const void* host, size_t bytes) {
@@ -3125,7 +3125,7 @@ static int sourcePassRing(Context* c, const DevSignals& srcSet, const DevSignals
     E3D_RET(premultipliedAdjoint(c, prem));
   }
   E3D_RET(choosePlan(c, L));
-  E3D_RET(ensureRing(c, c->srcRing, c->s0, c->s1, ringLevels(c)));  // anew if the rows changed
+  if (c->srcRing.empty()) E3D_RET(ensureRing(c, c->srcRing, c->s0, c->s1, ringLevels(c)));  // the rows changed
   c->tailReady = takesTail(c);
   c->pending = {};
   if (c->tailReady) E3D_RET(prepareInject(c, c->acqA, srcSet, false));

@@ -2820,6 +2820,7 @@ static int prepareCheckpoints(Context* c, int L, int& nseg) {
   nseg = (blocks + L - 1) / L;
   if (c->ckptSegLen != L || (int)c->ckpt.size() != nseg || c->ckptAllocType != c->ckptUsed ||
       c->vAllocType != c->vUsed) {
+    c->ckptSegLen = 0;  // until every buffer of the plan is there
     for (void* p : c->ckpt) devFree(c, p);
     for (float* p : c->ckptScale) devFree(c, p);
     c->ckpt.assign(nseg, nullptr);

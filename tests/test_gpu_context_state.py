@@ -389,3 +389,36 @@ def test_slabs_of_unlike_rows_equal_the_whole_grid(adjoint, surface):
     _equal(got, ref)
     sl.close()
     whole.close()
+
+
+def test_checkpoints_after_a_plan_that_ran_out_of_memory():
+    """A change of storage that found no memory for all its states is not taken for a plan in place: the
+    next forward makes the buffers that are missing."""
+    nz, nx, ny, nts = 72, 200, 400, 6
+    rng = np.random.default_rng(16)
+    med = _medium(nz, nx, ny)
+    sets = sp, so, rp, ro, sig = _device_sets(rng, nz, nx, ny, nts)
+    out = []
+    for short in (False, True):
+        pr = _propagator(nz, nx, ny, nts)
+        pr.set_medium(med)
+        pr.set_velocity_storage("fp32")
+        if short:
+            rec = torch.empty((nts, ro[9]), device="cuda")
+            pr.synchronize()
+            with _memory_left(1.15 * 18 * 4 * nz * nx * ny):
+                pr.step_only(0, 1)  # in unpadded rows from here on
+                pr.synchronize()
+            pr.set_checkpoint_policy("fp16", 2)
+            pr.fwi_forward_device(sp, so, rp, ro, sig, rec)
+            pr.synchronize()
+            pr.set_checkpoint_policy("fp32", 2)
+            with _memory_left(8 << 20):
+                with pytest.raises(N.E3DError, match="memory"):
+                    pr.fwi_forward_device(sp, so, rp, ro, sig, rec)
+                torch.cuda.synchronize()
+        pr.set_checkpoint_policy("fp32", 2)
+        out.append(_gradient(pr, sets, nts, ny, nx, nz))
+        assert pr.checkpoint_type == "fp32"
+        pr.close()
+    _equal(out[1], out[0])
